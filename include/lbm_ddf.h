@@ -59,9 +59,7 @@ extern "C" {
 
 /* step kernels (same results, different data movement) */
 #define LBM_KERNEL_AUTO 0      /* NODE (measured the fastest on B200) */
-#define LBM_KERNEL_NODE 1      /* one node per thread, any grid and side-wall mode (16-bit
-                                  storage with BGK collision: each node's update split
-                                  over two warps, each taking half the populations) */
+#define LBM_KERNEL_NODE 1      /* one node per thread, any grid and side-wall mode */
 #define LBM_KERNEL_ROW 2       /* whole x-rows staged by bulk copies; FP32 or FP64 storage,
                                   periodic sides, 32 <= LX <= 256, LX*element size a
                                   multiple of 16 bytes */
@@ -245,8 +243,7 @@ int lbm_selfcheck_division(int device, double divisor, uint64_t n, uint64_t seed
  * observables of every state the steps started from: out[i] is the state
  * after (initial step count + i) steps, as lbm_get_observables would report
  * it then.  Each step kernel reduces them from the moments it computes
- * anyway (in every storage format; for 16-bit BGK, half of each warp pair
- * of the split kernel), so the per-step observables cost no extra read of
+ * anyway (in every storage format), so the per-step observables cost no extra read of
  * the state (lbm_get_observables reads all populations once).  Call
  * lbm_get_observables for the state after the last step.  Node kernel only
  * (LBM_ERR_ARG if the case's step kernel is set to ROW); synchronises

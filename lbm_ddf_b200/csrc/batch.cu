@@ -52,6 +52,8 @@ template <class S> struct BatchCase {
     S *f_st, *g_st;      // the same arrays, for stores (see StepArgs)
     P *phip;
     uint32_t ps, nodes;
+    uint32_t ps_st;      // ps, for the 16-bit stores
+    uint32_t zero;       // 0 (see again())
     int32_t lx, ly, lz, swapped;
     FastDiv div_lx, div_ly;
     R tau, tauc, rcp_tau, rcp_tauc, rcp_rt;
@@ -70,24 +72,22 @@ template <class S> struct BatchCase {
     template <class I> __device__ __forceinline__ S &st(int which, int k, I j) const {
         return (which ? g_st : f_st)[((uint32_t)k * ps + (uint32_t)j) * elem_stride<S>()];
     }
-    // 16-bit storage: the (f_k, g_k) pair of node j as one 32-bit word
-    template <class I, class SS = S> __device__ __forceinline__ typename Pack16<SS>::T ld2(int k, I j) const {
-        return reinterpret_cast<const typename Pack16<SS>::T *>(f)[(uint32_t)k * ps + (uint32_t)j];
+    // 16-bit storage: address of the (f_k, g_k) pair of node j, one 32-bit word
+    template <class I, class SS = S> __device__ __forceinline__ const typename Pack16<SS>::T *ld2(int k, I j) const {
+        return reinterpret_cast<const typename Pack16<SS>::T *>(f) + ((uint32_t)k * ps + (uint32_t)j);
     }
-    template <class I, class SS = S> __device__ __forceinline__ typename Pack16<SS>::T &st2(int k, I j) const {
-        return reinterpret_cast<typename Pack16<SS>::T *>(f_st)[(uint32_t)k * ps + (uint32_t)j];
+    template <class I, class SS = S> __device__ __forceinline__ typename Pack16<SS>::T *st2(int k, I j) const {
+        return reinterpret_cast<typename Pack16<SS>::T *>(f_st) + ((uint32_t)k * ps_st + (uint32_t)j);
     }
 };
 
 // Resident threads per SM the batch kernel's registers are sized for: those
-// of the single-case kernel, except 512 (128 registers) for 16-bit storage:
-// one 256^3 FP16S case through the batch kernel on B200 ran at 15.7 GLUPS
-// with 640 threads (96 registers) and 19.2-20.9 with 512.
-template <class S> constexpr int batch_threads_per_sm() {
-    return sizeof(S) == 2 ? 512 : StepOccupancy<S>::value * 128;
-}
-template <class S, int BLOCK> struct BatchOccupancy {
-    static constexpr int value = batch_threads_per_sm<S>() / BLOCK > 0 ? batch_threads_per_sm<S>() / BLOCK : 1;
+// of the single-case kernel, except 640 (96 registers) for 16-bit BGK, which
+// holds 27 words beside the member's descriptor and spills at 768 (32-member
+// FP16S ensemble on B200: 21.5 GLUPS at 640, 17.1 at 768).
+template <class S, int BLOCK, int COLL> struct BatchOccupancy {
+    static constexpr int threads = sizeof(S) == 2 && COLL == LBM_COLLISION_BGK ? 640 : step_threads_per_sm<S>();
+    static constexpr int value = threads / BLOCK;
 };
 
 // Advances the members cases[0 .. ncases) of one group, all in layout
@@ -95,7 +95,7 @@ template <class S, int BLOCK> struct BatchOccupancy {
 // tile of member i (tile numbers are batch-wide; the group owns tiles
 // [tile_start[0], tile_start[ncases])).
 template <class S, int BLOCK, bool SWAPPED, int COLL>
-__global__ void __launch_bounds__(BLOCK, BatchOccupancy<S, BLOCK>::value)
+__global__ void __launch_bounds__(BLOCK, BatchOccupancy<S, BLOCK, COLL>::value)
     batch_step_kernel(const BatchCase<S> *__restrict__ cases, int ncases, const uint32_t *__restrict__ tile_start) {
     __shared__ uint32_t s_start[kMaxBatch + 1];
     for (int i = threadIdx.x; i <= ncases; i += BLOCK) s_start[i] = tile_start[i];
@@ -186,7 +186,7 @@ template <class S> BatchCase<S> describe(const lbm_case *c) {
     d.f = d.f_st = (S *)c->f;
     d.g = d.g_st = (S *)c->g;
     d.phip = (typename Codec<S>::P *)c->phip;
-    d.ps = (uint32_t)c->ps;
+    d.ps = d.ps_st = (uint32_t)c->ps;
     d.nodes = (uint32_t)c->nodes;
     d.lx = c->p.lx;
     d.ly = c->p.ly;

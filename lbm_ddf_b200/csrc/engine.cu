@@ -57,7 +57,6 @@ using namespace lbm_internal;
 namespace {
 constexpr int kObs = lbm::kObsTerms;   // partial sums per block (step.cuh add_obs_terms)
 constexpr int kObsThreads = 256;
-constexpr int kStepThreads = 128;
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -71,12 +70,11 @@ namespace lbm {
 //   9..11 phi on the planes iy = LY-1, LY-2, LY-3
 //   12 number of nodes with a non-finite moment
 //
-// split: the moments as the 16-bit BGK step kernel forms them (split_moments),
-// so these observables match those it reduces when it steps; else as the
-// node update forms them.
+// 16-bit storage: the moments as the step of collision model `coll` forms
+// them, so these observables match those it reduces when it steps.
 template <class S, bool SWAPPED, bool PERIODIC>
 __global__ void __launch_bounds__(kObsThreads) obs_kernel(const StepArgs<S> a, double *__restrict__ partial,
-                                                          int split) {
+                                                          int coll) {
     using R = typename Codec<S>::R;
     double acc[kObs];
 #pragma unroll
@@ -84,10 +82,12 @@ __global__ void __launch_bounds__(kObsThreads) obs_kernel(const StepArgs<S> a, d
     for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < a.nodes; n += gridDim.x * blockDim.x) {
         const Node g = make_node<PERIODIC>(a, n);
         if constexpr (elem_stride<S>() == 2) {
-            if (split) {
-                add_obs_terms(acc, split_moments<S, SWAPPED, PERIODIC>(a, g), g.iy, a.ly);
-                continue;
-            }
+            add_obs_terms(acc,
+                          coll == LBM_COLLISION_BGK
+                              ? step_moments16<S, SWAPPED, PERIODIC, LBM_COLLISION_BGK>(a, g)
+                              : step_moments16<S, SWAPPED, PERIODIC, LBM_COLLISION_REGULARIZED>(a, g),
+                          g.iy, a.ly);
+            continue;
         }
         R fr[Q], gr[Q];
         // rows away from the plates (and a closed box's z walls): no y or z
@@ -445,7 +445,8 @@ template <class S> StepArgs<S> make_args(const lbm_case *c) {
     }
     for (int b = 0; b < 3; b++)
         a.pairs[b] = a.pairs_st[b] = (S *)c->f + (size_t)(9 * b) * (size_t)c->ps * elem_stride<S>();
-    a.pair_row = (uint32_t)c->ps;
+    a.pair_row = a.pair_row_st = (uint32_t)c->ps;
+    a.zero = 0;
     a.obs_rows = nullptr;
     a.phip = (typename Codec<S>::P *)c->phip;
     a.lx = c->p.lx;
@@ -486,29 +487,16 @@ template <class Fn> int with_storage(const lbm_case *c, Fn &&fn) {
     return fail(LBM_ERR_ARG, "bad storage");
 }
 
-// Whether the case steps on step16_split_kernel (16-bit storage, BGK): 64
-// nodes per block there, 128 in step_kernel.
-bool split_step(const lbm_case *c) { return interleaved(c) && c->collision == LBM_COLLISION_BGK; }
-int step_blocks(const lbm_case *c) {
-    if (split_step(c)) return (int)grid_for(c->nodes, 64);
-    return (int)grid_for(c->nodes, c->p.storage == LBM_STORE_F32 ? node_threads<float>() : kStepThreads);
+int step_threads(const lbm_case *c) {
+    return c->p.storage == LBM_STORE_F64 ? node_threads<double>()
+           : c->p.storage == LBM_STORE_F32 ? node_threads<float>() : node_threads<__half>();
 }
-// rows of observables sums an observed step writes: one per warp of the node
-// kernel, one per warp pair of the 16-bit split kernel
-int obs_rows_of(const lbm_case *c) {
-    if (split_step(c)) return step_blocks(c) * 2;
-    return step_blocks(c) * ((c->p.storage == LBM_STORE_F32 ? node_threads<float>() : kStepThreads) / 32);
-}
+int step_blocks(const lbm_case *c) { return (int)grid_for(c->nodes, step_threads(c)); }
+// rows of observables sums an observed step writes: one per warp
+int obs_rows_of(const lbm_case *c) { return step_blocks(c) * (step_threads(c) / 32); }
 
 template <class S, bool SW, bool PER, bool OBS = false>
 void launch_step_t(const lbm_case *c, const StepArgs<S> &a, cudaStream_t st) {
-    // 16-bit storage, BGK: one node's update split over two warps
-    if constexpr (sizeof(S) == 2) {
-        if (c->collision == LBM_COLLISION_BGK) {
-            step16_split_kernel<S, SW, PER, OBS><<<grid_for(c->nodes, 64), 128, 0, st>>>(a);
-            return;
-        }
-    }
     constexpr int threads = node_threads<S>();
     const unsigned grid = grid_for(c->nodes, threads);
     if (c->collision == LBM_COLLISION_REGULARIZED)
@@ -617,13 +605,13 @@ template <class S, bool SW, bool PER> int obs_resident() {
     return resident;
 }
 template <class S>
-int launch_obs(const lbm_case *c, const StepArgs<S> &a, double *partial, int cap, int sms, int split,
+int launch_obs(const lbm_case *c, const StepArgs<S> &a, double *partial, int cap, int sms, int coll,
                cudaStream_t st) {
     const bool per = c->p.sides == LBM_SIDES_PERIODIC;
     const int resident = c->swapped ? (per ? obs_resident<S, true, true>() : obs_resident<S, true, false>())
                                     : (per ? obs_resident<S, false, true>() : obs_resident<S, false, false>());
     const int blocks = std::max(1, std::min(cap, sms * resident));
-    LBM_DISPATCH_LAYOUT(c, obs_kernel, blocks, kObsThreads, st, a, partial, split);
+    LBM_DISPATCH_LAYOUT(c, obs_kernel, blocks, kObsThreads, st, a, partial, coll);
     return blocks;
 }
 
@@ -934,7 +922,7 @@ int lbm_internal::enqueue_observables(const lbm_case *c, lbm_observables *dst, c
     return with_storage(c, [&](auto tag) {
         using S = std::remove_pointer_t<decltype(tag)>;
         const StepArgs<S> a = make_args<S>(c);
-        const int blocks = launch_obs<S>(c, a, c->partial, c->obs_blocks, c->sms, split_step(c) ? 1 : 0, st);
+        const int blocks = launch_obs<S>(c, a, c->partial, c->obs_blocks, c->sms, c->collision, st);
         ObsConsts k;
         k.nodes = (double)c->nodes;
         k.plane = (double)c->p.lx * (double)c->p.lz;
@@ -1000,14 +988,10 @@ static int step_observed(lbm_case *c, int32_t nsteps, lbm_observables *out, void
     if (nsteps == 0) return LBM_OK;
     DeviceGuard dg(c->p.device);
     cudaStream_t st = (cudaStream_t)stream;
-    // one row per warp of the node kernel (per warp pair of the 16-bit BGK
-    // kernel): room for the most rows, whichever kernel the case uses now
-    const int rows = obs_rows_of(c);
+    const int rows = obs_rows_of(c);   // one per warp of the node kernel
     const int parts = (rows + kRowChunk - 1) / kRowChunk;
-    const int max_rows = (int)grid_for(c->nodes, kStepThreads) * (kStepThreads / 32);
-    const int max_parts = (max_rows + kRowChunk - 1) / kRowChunk;
     if (!c->obs_rows) {   // per-warp rows, the chunk partials, the count of chunks done
-        const size_t bytes = (size_t)(max_rows + max_parts) * kObs * sizeof(double);
+        const size_t bytes = (size_t)(rows + parts) * kObs * sizeof(double);
         CUDA_TRY(cudaMalloc(&c->obs_rows, bytes + sizeof(double)));
         CUDA_TRY(cudaMemsetAsync((char *)c->obs_rows + bytes, 0, sizeof(double), st));
     }
@@ -1021,8 +1005,8 @@ static int step_observed(lbm_case *c, int32_t nsteps, lbm_observables *out, void
         CUDA_TRY(cudaMalloc(&c->obs_series, (size_t)nsteps * sizeof(lbm_observables)));
         c->obs_series_cap = nsteps;
     }
-    double *partial = c->obs_rows + (size_t)max_rows * kObs;
-    unsigned *done = (unsigned *)(partial + (size_t)max_parts * kObs);
+    double *partial = c->obs_rows + (size_t)rows * kObs;
+    unsigned *done = (unsigned *)(partial + (size_t)parts * kObs);
     rc = with_storage(c, [&](auto tag) {
         using S = std::remove_pointer_t<decltype(tag)>;
         StepArgs<S> a = make_args<S>(c);
@@ -1256,8 +1240,8 @@ int lbm_observables_noalloc(const lbm_params *p, const void *f, const void *g, c
         using S = std::remove_pointer_t<decltype(tag)>;
         const StepArgs<S> a = make_args<S>(&view);
         const lbm_case *c = &view;
-        // 16-bit storage: the moments as the BGK step kernel forms them
-        const int blocks = launch_obs<S>(c, a, scratch, cap, sms, interleaved(c) ? 1 : 0, st);
+        // 16-bit storage: the moments as the BGK step forms them
+        const int blocks = launch_obs<S>(c, a, scratch, cap, sms, LBM_COLLISION_BGK, st);
         ObsConsts k;
         k.nodes = (double)nodes;
         k.plane = (double)p->lx * (double)p->lz;

@@ -94,25 +94,26 @@ template <class S> struct StepArgs {
         if constexpr (elem_stride<S>() == 1) return st_row(which, k)[j];
         else return st_row(which, k)[2u * (uint32_t)j];
     }
-    // 16-bit storage: the (f_k, g_k) pair of node j as one 32-bit word.
-    // The pair array is addressed in three blocks of nine rows, pair
-    // (k mod 9) * pair_row + j of block k / 9, with a 32-bit index (one
-    // multiply-add and one wide add per access; on B200 this ran 18% faster
-    // than the per-row bases above, which FP32 and FP64 keep: for them the
-    // same indexing measured within 1%).  The index stays below
-    // 9 pair_row < 2^32 for every case the C ABI accepts in 16-bit storage.
-    template <class I, class SS = S> __device__ __forceinline__ typename Pack16<SS>::T ld2(int k, I j) const {
-        return reinterpret_cast<const typename Pack16<SS>::T *>(pairs[k / 9])[(uint32_t)(k % 9) * pair_row +
-                                                                              (uint32_t)j];
+    // 16-bit storage: address of the (f_k, g_k) pair of node j, one 32-bit
+    // word, for the loads (ld2) and the stores (st2).  The pair array is
+    // addressed in three blocks of nine rows, pair (k mod 9) * pair_row + j
+    // of block k / 9, with a 32-bit index (one multiply-add and one wide add
+    // per access).  The index stays below 9 pair_row < 2^32 for every case
+    // the C ABI accepts in 16-bit storage.
+    template <class I, class SS = S> __device__ __forceinline__ const typename Pack16<SS>::T *ld2(int k, I j) const {
+        return reinterpret_cast<const typename Pack16<SS>::T *>(pairs[k / 9]) +
+               ((uint32_t)(k % 9) * pair_row + (uint32_t)j);
     }
-    template <class I, class SS = S> __device__ __forceinline__ typename Pack16<SS>::T &st2(int k, I j) const {
-        return reinterpret_cast<typename Pack16<SS>::T *>(pairs_st[k / 9])[(uint32_t)(k % 9) * pair_row +
-                                                                           (uint32_t)j];
+    template <class I, class SS = S> __device__ __forceinline__ typename Pack16<SS>::T *st2(int k, I j) const {
+        return reinterpret_cast<typename Pack16<SS>::T *>(pairs_st[k / 9]) +
+               ((uint32_t)(k % 9) * pair_row_st + (uint32_t)j);
     }
     double *obs_rows;  // fused observables: one row of kObsTerms sums per warp (else unused)
     S *pairs[3];       // 16-bit storage: rows 0, 9 and 18 of the (f, g) pair array
     S *pairs_st[3];    // the same, for the stores (see fs)
     uint32_t pair_row; // pairs per row (the padded node count)
+    uint32_t pair_row_st;  // the same, for the stores
+    uint32_t zero;         // 0 (see again())
 };
 
 // Geometry of one node: coordinates, and node-index displacements to the
@@ -212,8 +213,7 @@ template <bool PERIODIC> __device__ __forceinline__ bool yz_interior(const Node 
 // (decided over the warp, so a warp takes one path), else kNoneInside.
 // In the natural layout every access is at the node itself, so kAllInside
 // would compile to kRowInside's code again: with SWAPPED false it is not
-// returned, which keeps a third copy of the update out of the kernel (in the
-// issue-bound 16-bit split kernel a larger body measured slower).
+// returned, which keeps a third copy of the update out of the kernel.
 template <bool PERIODIC, bool SWAPPED = true> __device__ __forceinline__ int node_path(const Node &g) {
     if (!yz_interior<PERIODIC>(g)) return kNoneInside;
     if constexpr (!PERIODIC && SWAPPED) {
@@ -222,9 +222,7 @@ template <bool PERIODIC, bool SWAPPED = true> __device__ __forceinline__ int nod
     return kRowInside;
 }
 // node_path, with a closed box's warps at one x wall told apart (kRowLoWall,
-// kRowHiWall), for updates that take those paths (the node kernel's swapped
-// layout; in the 16-bit split kernel the two extra paths measured 12% slower
-// on the swapped closed-box step).
+// kRowHiWall), for the FP32 and FP64 updates of the swapped layout.
 template <bool PERIODIC> __device__ __forceinline__ int node_path_x(const Node &g) {
     if (!yz_interior<PERIODIC>(g)) return kNoneInside;
     if constexpr (!PERIODIC) {
@@ -253,15 +251,25 @@ __device__ __forceinline__ S load_pop(const A &a, const Node &g) {
     return *(in ? a.ldp(WHICH, opp(K), (int32_t)g.n + disp<DX, DY, DZ>(g)) : a.ldp(WHICH, K, g.n));
 }
 
+// Whether population K of a 16-bit node takes its address by a select
+// between the neighbour and the node itself: the x-moving populations of a
+// closed box's rows (see update_node16).  Elsewhere the test is a constant or
+// rare, and a branch.
+template <bool SWAPPED, bool PERIODIC, int INTERIOR, int K> constexpr bool selects_address() {
+    return SWAPPED && !PERIODIC && INTERIOR == kRowInside && cx(K) != 0;
+}
+
 // The (f_k, g_k) pair that node g collides in this step, as load_pop finds
-// each value, with one 32-bit load.  (Here a branch: the address select of
-// load_pop measured 3% slower in the 16-bit closed-box swapped step.)
-template <class S, bool SWAPPED, int K, int INTERIOR, class A>
+// each value, with one 32-bit load.
+template <class S, bool SWAPPED, bool PERIODIC, int K, int INTERIOR, class A>
 __device__ __forceinline__ typename Pack16<S>::T load_pair(const A &a, const Node &g) {
-    if (!SWAPPED) return a.ld2(K, g.n);
+    if (!SWAPPED) return *a.ld2(K, g.n);
     constexpr int DX = -cx(K), DY = -cy(K), DZ = -cz(K);
-    if (inside_t<INTERIOR, DX, DY, DZ>(g)) return a.ld2(opp(K), (int32_t)g.n + disp<DX, DY, DZ>(g));
-    return a.ld2(K, g.n);
+    const bool in = inside_t<INTERIOR, DX, DY, DZ>(g);
+    if constexpr (selects_address<SWAPPED, PERIODIC, INTERIOR, K>())
+        return *(in ? a.ld2(opp(K), (int32_t)g.n + disp<DX, DY, DZ>(g)) : a.ld2(K, g.n));
+    if (in) return *a.ld2(opp(K), (int32_t)g.n + disp<DX, DY, DZ>(g));
+    return *a.ld2(K, g.n);
 }
 
 // 16-bit storage keeps g_i / w_i - T_c at every location, T_c(iy) =
@@ -286,13 +294,6 @@ __device__ __forceinline__ float read_shift_delta(const A &a, const Node &g) {
     if constexpr (!SWAPPED || DY == 0) return 0.f;
     else return inside_t<INTERIOR, DX, DY, DZ>(g) ? (float)cy(K) * (float)a.t_dy : 0.f;
 }
-template <bool SWAPPED, int I, int INTERIOR, class A>
-__device__ __forceinline__ float write_shift_delta(const A &a, const Node &g) {
-    constexpr int DX = cx(I), DY = cy(I), DZ = cz(I);
-    if constexpr (!SWAPPED || DY == 0) return 0.f;
-    else return inside_t<INTERIOR, DX, DY, DZ>(g) ? (float)cy(I) * (float)a.t_dy : 0.f;
-}
-
 template <class S, bool SWAPPED, int INTERIOR = kNoneInside, class A>
 __device__ __forceinline__ void gather(const A &a, const Node &g, typename Codec<S>::R (&fr)[Q],
                                        typename Codec<S>::R (&gr)[Q]) {
@@ -306,7 +307,7 @@ __device__ __forceinline__ void gather(const A &a, const Node &g, typename Codec
             // the moment sums in one kernel and not in another, so every
             // kernel that gathers (the step, the observables) forms the same
             // FP32 moments
-            const float2 v = Pack16<S>::unpack(load_pair<S, SWAPPED, K, INTERIOR>(a, g));
+            const float2 v = Pack16<S>::unpack(load_pair<S, SWAPPED, false, K, INTERIOR>(a, g));
             fr[K] = __fmul_rn((float)wd(K), v.x);
             gr[K] = __fmul_rn((float)wd(K), __fadd_rn(v.y, __fadd_rn(s0, read_shift_delta<SWAPPED, K, INTERIOR>(a, g))));
         } else {
@@ -574,8 +575,6 @@ __device__ __forceinline__ void scatter(const A &a, const Node &g, const typenam
                                         const typename Codec<S>::R (&gr)[Q], typename Codec<S>::R rho) {
     using C = Codec<S>;
     using R = typename C::R;
-    float s0 = 0.f;
-    if constexpr (elem_stride<S>() == 2) s0 = shift0(a, g);
     Unroll<0, Q>::run([&](auto ii) {
         constexpr int I = decltype(ii)::value;
         constexpr int DX = cx(I), DY = cy(I), DZ = cz(I);
@@ -584,15 +583,8 @@ __device__ __forceinline__ void scatter(const A &a, const Node &g, const typenam
         const bool out_y = INTERIOR == kNoneInside && ((DY < 0 && !g.vym) || (DY > 0 && !g.vyp));
         const bool out_z = !PERIODIC && INTERIOR == kNoneInside && ((DZ < 0 && !g.vzm) || (DZ > 0 && !g.vzp));
         if (DY != 0 && out_y && !out_z) gv = abb<I>(gv, DY < 0 ? a.t_hot : a.t_cold, rho);
-        if constexpr (elem_stride<S>() == 2) {   // (f, g) pairs: f/w and g/w - T_c at the location, packed
-            // the location's T_c is s0 - write_shift_delta (it is s0 at the node itself)
-            const float sl = s0 - write_shift_delta<SWAPPED, I, INTERIOR>(a, g);
-            const auto v = Pack16<S>::pack(fv * (float)winv(I), fmaf(gv, (float)winv(I), -sl));
-            if (SWAPPED && inside_t<INTERIOR, DX, DY, DZ>(g))
-                a.st2(I, (int32_t)g.n + disp<DX, DY, DZ>(g)) = v;
-            else
-                a.st2(opp(I), g.n) = v;
-        } else {
+        static_assert(elem_stride<S>() == 1, "16-bit pairs are stored by put_pair");
+        {
             // to the neighbour x + c_I (swapped layout, inside) or back to
             // the node itself, the address chosen by a select (see load_pop)
             const bool in = SWAPPED && inside_t<INTERIOR, DX, DY, DZ>(g);
@@ -603,22 +595,25 @@ __device__ __forceinline__ void scatter(const A &a, const Node &g, const typenam
     });
 }
 
-// Resident 128-thread blocks per SM the register allocation is sized for:
-// 3 (<= 168 registers) for FP64, which holds 54 doubles across the
-// collision (B200, 256^3: 6.7, 7.4 and 6.6 GLUPS at 2, 3 and 4 blocks, the
-// last spilling); 4 (<= 128) for FP32 and 16-bit storage (256^3 FP16S with
-// interleaved pairs: 21.7 GLUPS at 4 blocks, 14.2 at 5 and 14.6 at 6, where
-// the update spills).
-template <class S> struct StepOccupancy {
-    static constexpr int value = sizeof(S) == 8 ? 3 : 4;
-};
-// Threads per block of step_kernel: FP32 steps in blocks of two warps (a
-// block holds its SM slot until its slowest warp is done, and two-warp
-// blocks waste less of it: B200, 256^3, natural layout -1.8%, closed-box
-// swapped -3.6%); FP64 measured 3% slower so and keeps four, as does 16-bit
-// storage with the regularised collision (not measured).  The register
-// budget is the same: StepOccupancy x 128 threads per SM.
-template <class S> constexpr int node_threads() { return std::is_same<S, float>::value ? 64 : 128; }
+// Threads per block of step_kernel: FP32 and 16-bit steps in blocks of two
+// warps (a block holds its SM slot until its slowest warp is done, and
+// two-warp blocks waste less of it: B200, 256^3 FP32, natural layout -1.8%,
+// closed-box swapped -3.6%; FP16S BGK closed-box swapped 640 against 667 for
+// the pair of layouts); FP64 measured 3% slower so and keeps four.
+template <class S> __host__ __device__ constexpr int node_threads() { return sizeof(S) == 8 ? 128 : 64; }
+// Resident threads per SM the register allocation is sized for: 384 (<= 168
+// registers) for FP64, which holds 54 doubles across the collision (B200,
+// 256^3: 6.7, 7.4 and 6.6 GLUPS at 256, 384 and 512 threads, the last
+// spilling); 512 (<= 128) for FP32; 768 (80) for 16-bit storage, which holds
+// 27 packed words (256^3 FP16S, periodic, both layouts summed: BGK 1207 us at
+// 768 threads, 1272 at 640, over 2500 at 896 where the rows' body spills;
+// regularised 1390 at 768 and 1440 at 640).
+template <class S> __host__ __device__ constexpr int step_threads_per_sm() {
+    return sizeof(S) == 8 ? 384 : sizeof(S) == 4 ? 512 : 768;
+}
+// The step kernel's launch bounds (FP32's are stated for blocks of 128, the
+// same register budget).
+template <class S> constexpr int bound_threads() { return sizeof(S) == 2 ? node_threads<S>() : 128; }
 
 // The whole update of one node: gather, moments, collision, carried
 // temperature, scatter.
@@ -699,301 +694,36 @@ template <class R> struct NodeOut {
 //
 // FP16S / BF16S rows hold (fh_i, gh_i) pairs, fh_i = f_i / w_i and
 // gh_i = g_i / w_i - T_c (T_c the conduction profile at the location, see
-// shift0), one 32-bit word per population and node.  The
-// update below works on those directly (FP32 arithmetic): the moments sum
-// them per weight class and weight the four class sums, and the BGK steps in
-// normalised form,
-//   fh*_i = fh_i - (fh_i - (rho + p_i)) / tau + 3 (1 - 1/(2 tau)) F_y (c_iy - u_y) (1 + p_i)
-//   gh*_i = gh_i - (gh_i + t0 - phi (1 + p_i)) / tau_c,
-// p_i = 3 c_i.u + 4.5 (c_i.u)^2 - 1.5 u^2, need no weight on load or store.
-// Opposite directions share c.u and the quadratic part of p.  The same
-// update as collide_fast, with fewer instructions per node.
+// shift0), one 32-bit word per population and node.  The updates below work
+// on those directly in FP32, one node per thread.  A thread first loads its
+// 27 words, all of them before the first is unpacked, so that they are in
+// flight together and held in one register each; it sums the moments, then
+// relaxes and stores pair by pair.  What bounds these kernels is memory
+// latency, and two things decide how well it is hidden:
+//  - nothing should be loaded between the stores.  Reading each pair a second
+//    time (from L1) instead of holding it ran at a third of the speed, and
+//    builds whose registers spilled there at half to two thirds.  So the
+//    register budget is the one at which the rows' body hardly spills, not
+//    the smallest;
+//  - the registers must go to the 27 words.  The 26 neighbour indices of the
+//    loads are the stores' again; again() keeps them from being held.
+// Warps are retired in blocks of two (a block holds its SM slot until its
+// slowest warp is done).
 
-template <class S, bool SWAPPED, bool PERIODIC, int INTERIOR, class A>
-__device__ __forceinline__ void gather_norm(const A &a, const Node &g, float2 (&fg)[Q]) {
-    Unroll<0, Q>::run([&](auto kk) {
-        constexpr int K = decltype(kk)::value;
-        fg[K] = Pack16<S>::unpack(load_pair<S, SWAPPED, K, INTERIOR>(a, g));
-        // relative to the node's T_c; on interior rows of a periodic box in
-        // the swapped layout the read and write re-referencing is folded
-        // into the collision (collide_norm's `fold`), as the moments do not
-        // see it (the deltas of each weight class sum to zero); a closed
-        // box's x walls keep some populations in the node's own plane, so
-        // there each delta is applied
-        if constexpr (!(SWAPPED && all_inside<INTERIOR, PERIODIC>())) fg[K].y += read_shift_delta<SWAPPED, K, INTERIOR>(a, g);
-    });
+// Node g for the stores: the same node, formed from a zero that the compiler
+// cannot see, so that it forms the stores' addresses anew.
+template <class A> __device__ __forceinline__ Node again(const A &a, const Node &g) {
+    Node s = g;
+    s.n += a.zero;
+    s.dxm += a.zero;
+    s.dxp += a.zero;
+    s.dzm += a.zero;
+    s.dzp += a.zero;
+    return s;
 }
 
-// fg[i] = (fh_i, gh_i); gh here is g/w - s0 (s0 the node's conduction-profile temperature); t0 is
-// the mean temperature of the force term.
-__device__ __forceinline__ Moments<float> moments_norm(const float2 (&fg)[Q], float phip, float gbeta, float t0,
-                                                       float s0) {
-    float2 rt[4] = {};   // (sum fh, sum gh) per weight class, paired
-    float x[4] = {0.f, 0.f, 0.f, 0.f}, y[4] = {0.f, 0.f, 0.f, 0.f}, z[4] = {0.f, 0.f, 0.f, 0.f};
-    Unroll<0, Q>::run([&](auto kk) {
-        constexpr int K = decltype(kk)::value;
-        constexpr int C = wclass(K);
-        rt[C] = add2(rt[C], fg[K]);
-        if (cx(K) > 0) x[C] += fg[K].x;
-        if (cx(K) < 0) x[C] -= fg[K].x;
-        if (cy(K) > 0) y[C] += fg[K].x;
-        if (cy(K) < 0) y[C] -= fg[K].x;
-        if (cz(K) > 0) z[C] += fg[K].x;
-        if (cz(K) < 0) z[C] -= fg[K].x;
-    });
-    const float w0 = (float)wd(0), w1 = (float)wd(1), w2 = (float)wd(7), w3 = (float)wd(19);
-    Moments<float> m;
-    const float2 s = fma2(splat(w3), rt[3], fma2(splat(w2), rt[2], fma2(splat(w1), rt[1], mul2(splat(w0), rt[0]))));
-    m.rho = s.x;
-    m.ux = fmaf(w3, x[3], fmaf(w2, x[2], w1 * x[1]));
-    const float jy = fmaf(w3, y[3], fmaf(w2, y[2], w1 * y[1]));
-    m.uz = fmaf(w3, z[3], fmaf(w2, z[2], w1 * z[1]));
-    m.phi = s.y + s0;   // sum w_i (gh_i + s0)
-    m.uy = jy + 0.5f * (gbeta * (phip - t0));
-    return m;
-}
-
-// Both relaxations as affine maps of the old value, with per-node
-// coefficients (k = kf (c_y - u_y) takes three values, one per c_y):
-//   fh* = (1 - om_f) fh + (om_f rho + k) + (om_f + k) p
-//   gh* = (1 - om_g) gh + om_g (phi - s0) + om_g phi p
-// and p_I, p_J = (q +/- 2 eu) / 2 with q = eu^2 - 3 u^2 for a pair of
-// opposite directions: two multiply-adds per population and three per pair.
-// (gh = g/w - s0; t0 enters only the buoyancy force.)  fold: the plane
-// spacing of the conduction profile when gh holds raw stored values that
-// were read from, and go to, the planes y - c_y and y + c_y (interior rows
-// of a periodic box, swapped layout): ag (v + c_y fold) + ... + c_y fold = ag v + ... +
-// (ag + 1) c_y fold, one more coefficient per c_y; else 0.
-__device__ __forceinline__ void collide_norm(float2 (&fg)[Q], const Moments<float> &m, float om_f, float om_g,
-                                             float force_fac, float gbeta, float t0, float s0, float fold) {
-    const float ux3 = 3.f * m.ux, uy3 = 3.f * m.uy, uz3 = 3.f * m.uz;
-    const float uv = 3.f * (m.ux * m.ux + m.uy * m.uy + m.uz * m.uz);
-    const float kf = 3.f * force_fac * (gbeta * (m.phi - t0));
-    const float k_m = kf * (-1.f - m.uy), k_0 = kf * (-m.uy), k_p = kf * (1.f - m.uy);
-    const float af = 1.f - om_f, orho = om_f * m.rho;
-    const float c0[3] = {orho + k_m, orho + k_0, orho + k_p};    // indexed by c_y + 1
-    const float c1[3] = {om_f + k_m, om_f + k_0, om_f + k_p};
-    const float ag = 1.f - om_g, d1 = om_g * m.phi, d0 = om_g * (m.phi - s0);
-    const float df = (ag + 1.f) * fold;
-    const float d0c[3] = {d0 - df, d0, d0 + df};                    // indexed by c_y + 1
-    // (fh, gh) <- (af fh + c1 p + c0, ag gh + d1 p + d0c): both at once
-    const float2 a2 = make_float2(af, ag);
-    auto relax = [&](float2 &v, float p, int cy1) {
-        v = fma2(a2, v, fma2(make_float2(c1[cy1], d1), splat(p), make_float2(c0[cy1], d0c[cy1])));
-    };
-    relax(fg[0], -0.5f * uv, 1);
-    Unroll<1, Q>::run([&](auto ii) {
-        constexpr int I = decltype(ii)::value;
-        constexpr int J = opp(I);
-        if constexpr (I < J) {
-            float eu = 0.f;
-            if (cx(I) > 0) eu += ux3;
-            if (cx(I) < 0) eu -= ux3;
-            if (cy(I) > 0) eu += uy3;
-            if (cy(I) < 0) eu -= uy3;
-            if (cz(I) > 0) eu += uz3;
-            if (cz(I) < 0) eu -= uz3;
-            const float q = fmaf(eu, eu, -uv);
-            relax(fg[I], fmaf(0.5f, q, eu), cy(I) + 1);
-            relax(fg[J], fmaf(0.5f, q, -eu), cy(J) + 1);
-        }
-    });
-}
-
-// scatter() for the normalised variables: anti-bounce-back in normalised
-// form, gh' = 2 T_wall (1 + rho) - gh* - 2 t0, no weights on store, and one
-// 32-bit store of the packed (f, g) pair per population.
-template <class S, bool SWAPPED, bool PERIODIC, int INTERIOR, class A>
-__device__ __forceinline__ void scatter_norm(const A &a, const Node &g, const float2 (&fg)[Q], float rho, float s0) {
-    Unroll<0, Q>::run([&](auto ii) {
-        constexpr int I = decltype(ii)::value;
-        constexpr int DX = cx(I), DY = cy(I), DZ = cz(I);
-        float gv = fg[I].y;
-        const bool out_y = INTERIOR == kNoneInside && ((DY < 0 && !g.vym) || (DY > 0 && !g.vyp));
-        const bool out_z = !PERIODIC && INTERIOR == kNoneInside && ((DZ < 0 && !g.vzm) || (DZ > 0 && !g.vzp));
-        if (DY != 0 && out_y && !out_z) gv = 2.f * (DY < 0 ? a.t_hot : a.t_cold) * (1.f + rho) - gv - 2.f * s0;
-        // relative to T_c at the location written (folded into the
-        // collision on interior rows of a periodic box's swapped layout)
-        if constexpr (!(SWAPPED && all_inside<INTERIOR, PERIODIC>())) gv += write_shift_delta<SWAPPED, I, INTERIOR>(a, g);
-        const typename Pack16<S>::T v = Pack16<S>::pack(fg[I].x, gv);
-        if (SWAPPED && inside_t<INTERIOR, DX, DY, DZ>(g))
-            a.st2(I, (int32_t)g.n + disp<DX, DY, DZ>(g)) = v;
-        else
-            a.st2(opp(I), g.n) = v;
-    });
-}
-
-template <class S, bool SWAPPED, bool PERIODIC, class A>
-__device__ __forceinline__ NodeOut<float> update_node_norm(const A &a, uint32_t n) {
-    const Node g = make_node<PERIODIC>(a, n);
-    float2 fg[Q];
-    const int path = node_path<PERIODIC, SWAPPED>(g);
-    if (path == kRowInside)
-        gather_norm<S, SWAPPED, PERIODIC, kRowInside>(a, g, fg);
-    else if (SWAPPED && !PERIODIC && path == kAllInside)
-        gather_norm<S, SWAPPED, PERIODIC, PERIODIC ? kRowInside : kAllInside>(a, g, fg);
-    else
-        gather_norm<S, SWAPPED, PERIODIC, kNoneInside>(a, g, fg);
-    const float s0 = shift0(a, g);
-    Moments<float> m = moments_norm(fg, a.phip[n], a.gb, a.t0, s0);
-    if (a.use_phi_fix) m.phi = a.phi_fix;
-    const bool fold = SWAPPED && (path == kAllInside || (PERIODIC && path == kRowInside));
-    collide_norm(fg, m, a.omega_f, a.omega_g, a.force_fac, a.gb, a.t0, s0, fold ? (float)a.t_dy : 0.f);
-    a.phip[n] = m.phi;
-    if (path == kRowInside)
-        scatter_norm<S, SWAPPED, PERIODIC, kRowInside>(a, g, fg, m.rho, s0);
-    else if (SWAPPED && !PERIODIC && path == kAllInside)
-        scatter_norm<S, SWAPPED, PERIODIC, PERIODIC ? kRowInside : kAllInside>(a, g, fg, m.rho, s0);
-    else
-        scatter_norm<S, SWAPPED, PERIODIC, kNoneInside>(a, g, fg, m.rho, s0);
-    return {m, g.iy};
-}
-
-// ---- 16-bit storage, BGK: one node's update split over two warps ----------
-//
-// The one-node update is latency-bound: a warp has its loads outstanding
-// only before its long update.  Here two warps share 32 nodes: half 0 loads,
-// relaxes and stores the rest population and the opposite pairs (1,3) (2,4)
-// (5,6) (7,9) (19,25) (20,26), half 1 the other seven pairs.  Each sums the
-// moments of its populations; the two exchange the five partial sums through
-// shared memory under a two-warp barrier and add them (addition commutes
-// exactly, so both hold the same moments).  A thread holds 13-14 pairs
-// instead of 27, so twice the warps are resident, and each warp's update
-// between its load phases is half as long.  The halves are chosen by warp
-// index, so no warp diverges.
-
-__host__ __device__ constexpr int pair_rep(int k) { return k < opp(k) ? k : opp(k); }
-// the half of the split update that owns population k
-__host__ __device__ constexpr int half_of(int k) {
-    return (k == 0 || pair_rep(k) == 1 || pair_rep(k) == 2 || pair_rep(k) == 5 || pair_rep(k) == 7 ||
-            pair_rep(k) == 19 || pair_rep(k) == 20)
-               ? 0
-               : 1;
-}
-
-// Every population in exactly one half, opposite pairs together (the
-// in-place update of a pair's two locations stays within one warp), 13 and
-// 14 populations.
-__host__ __device__ constexpr bool split_halves_ok() {
-    int n0 = 0;
-    for (int k = 0; k < Q; k++) {
-        if (half_of(k) != 0 && half_of(k) != 1) return false;
-        if (half_of(k) != half_of(opp(k))) return false;
-        n0 += half_of(k) == 0;
-    }
-    return n0 == 13 && half_of(0) == 0;
-}
-static_assert(split_halves_ok(), "split update: bad population halves");
-
-template <int H, class S, bool SWAPPED, bool PERIODIC, int INTERIOR, class A>
-__device__ __forceinline__ void gather_half(const A &a, const Node &g, float2 (&fg)[Q]) {
-    Unroll<0, Q>::run([&](auto kk) {
-        constexpr int K = decltype(kk)::value;
-        if constexpr (half_of(K) == H) {
-            fg[K] = Pack16<S>::unpack(load_pair<S, SWAPPED, K, INTERIOR>(a, g));
-            if constexpr (!(SWAPPED && all_inside<INTERIOR, PERIODIC>())) fg[K].y += read_shift_delta<SWAPPED, K, INTERIOR>(a, g);
-        }
-    });
-}
-
-// The half's share of rho, j_x, j_y, j_z and sum w_i gh_i (as moments_norm);
-// the (rho, phi) class sums and their weighting as paired FP32 operations
-template <int H> __device__ __forceinline__ void partial_moments(const float2 (&fg)[Q], float (&p)[5]) {
-    float2 rt[4] = {};   // (sum fh, sum gh) per weight class
-    float x[4] = {0.f, 0.f, 0.f, 0.f}, y[4] = {0.f, 0.f, 0.f, 0.f}, z[4] = {0.f, 0.f, 0.f, 0.f};
-    Unroll<0, Q>::run([&](auto kk) {
-        constexpr int K = decltype(kk)::value;
-        if constexpr (half_of(K) == H) {
-            constexpr int C = wclass(K);
-            rt[C] = add2(rt[C], fg[K]);
-            if (cx(K) > 0) x[C] += fg[K].x;
-            if (cx(K) < 0) x[C] -= fg[K].x;
-            if (cy(K) > 0) y[C] += fg[K].x;
-            if (cy(K) < 0) y[C] -= fg[K].x;
-            if (cz(K) > 0) z[C] += fg[K].x;
-            if (cz(K) < 0) z[C] -= fg[K].x;
-        }
-    });
-    const float w0 = (float)wd(0), w1 = (float)wd(1), w2 = (float)wd(7), w3 = (float)wd(19);
-    const float2 s = fma2(splat(w3), rt[3], fma2(splat(w2), rt[2], fma2(splat(w1), rt[1], mul2(splat(w0), rt[0]))));
-    p[0] = s.x;
-    p[1] = fmaf(w3, x[3], fmaf(w2, x[2], w1 * x[1]));
-    p[2] = fmaf(w3, y[3], fmaf(w2, y[2], w1 * y[1]));
-    p[3] = fmaf(w3, z[3], fmaf(w2, z[2], w1 * z[1]));
-    p[4] = s.y;
-}
-
-// collide_norm for the half's populations
-template <int H>
-__device__ __forceinline__ void collide_half(float2 (&fg)[Q], const Moments<float> &m, float om_f, float om_g,
-                                             float force_fac, float gbeta, float t0, float s0, float fold) {
-    const float ux3 = 3.f * m.ux, uy3 = 3.f * m.uy, uz3 = 3.f * m.uz;
-    const float uv = 3.f * (m.ux * m.ux + m.uy * m.uy + m.uz * m.uz);
-    const float kf = 3.f * force_fac * (gbeta * (m.phi - t0));
-    const float k_m = kf * (-1.f - m.uy), k_0 = kf * (-m.uy), k_p = kf * (1.f - m.uy);
-    const float af = 1.f - om_f, orho = om_f * m.rho;
-    const float c0[3] = {orho + k_m, orho + k_0, orho + k_p};
-    const float c1[3] = {om_f + k_m, om_f + k_0, om_f + k_p};
-    const float ag = 1.f - om_g, d1 = om_g * m.phi, d0 = om_g * (m.phi - s0);
-    const float df = (ag + 1.f) * fold;
-    const float d0c[3] = {d0 - df, d0, d0 + df};
-    // (fh, gh) <- (af fh + c1 p + c0, ag gh + d1 p + d0c): both at once
-    const float2 a2 = make_float2(af, ag);
-    auto relax = [&](float2 &v, float p, int cy1) {
-        v = fma2(a2, v, fma2(make_float2(c1[cy1], d1), splat(p), make_float2(c0[cy1], d0c[cy1])));
-    };
-    if constexpr (H == 0) relax(fg[0], -0.5f * uv, 1);
-    Unroll<1, Q>::run([&](auto ii) {
-        constexpr int I = decltype(ii)::value;
-        constexpr int J = opp(I);
-        if constexpr (I < J && half_of(I) == H) {
-            float eu = 0.f;
-            if (cx(I) > 0) eu += ux3;
-            if (cx(I) < 0) eu -= ux3;
-            if (cy(I) > 0) eu += uy3;
-            if (cy(I) < 0) eu -= uy3;
-            if (cz(I) > 0) eu += uz3;
-            if (cz(I) < 0) eu -= uz3;
-            const float q = fmaf(eu, eu, -uv);
-            relax(fg[I], fmaf(0.5f, q, eu), cy(I) + 1);
-            relax(fg[J], fmaf(0.5f, q, -eu), cy(J) + 1);
-        }
-    });
-}
-
-// scatter_norm for the half's populations
-template <int H, class S, bool SWAPPED, bool PERIODIC, int INTERIOR, class A>
-__device__ __forceinline__ void scatter_half(const A &a, const Node &g, const float2 (&fg)[Q], float rho, float s0) {
-    Unroll<0, Q>::run([&](auto ii) {
-        constexpr int I = decltype(ii)::value;
-        if constexpr (half_of(I) == H) {
-            constexpr int DX = cx(I), DY = cy(I), DZ = cz(I);
-            float gv = fg[I].y;
-            const bool out_y = INTERIOR == kNoneInside && ((DY < 0 && !g.vym) || (DY > 0 && !g.vyp));
-            const bool out_z = !PERIODIC && INTERIOR == kNoneInside && ((DZ < 0 && !g.vzm) || (DZ > 0 && !g.vzp));
-            if (DY != 0 && out_y && !out_z) gv = 2.f * (DY < 0 ? a.t_hot : a.t_cold) * (1.f + rho) - gv - 2.f * s0;
-            if constexpr (!(SWAPPED && all_inside<INTERIOR, PERIODIC>())) gv += write_shift_delta<SWAPPED, I, INTERIOR>(a, g);
-            const typename Pack16<S>::T v = Pack16<S>::pack(fg[I].x, gv);
-            if (SWAPPED && inside_t<INTERIOR, DX, DY, DZ>(g))
-                a.st2(I, (int32_t)g.n + disp<DX, DY, DZ>(g)) = v;
-            else
-                a.st2(opp(I), g.n) = v;
-        }
-    });
-}
-
-// Waits until both warps of warp pair `pair` (0 or 1; 64 threads) arrive,
-// on named barrier 1 + pair (immediate ids, so the block reserves three
-// barriers); the non-aligned form, so lanes need not be converged.
-__device__ __forceinline__ void pair_barrier(int pair) {
-    if (pair == 0)
-        asm volatile("barrier.sync 1, 64;\n" ::: "memory");
-    else
-        asm volatile("barrier.sync 2, 64;\n" ::: "memory");
-}
-
-// Receives a node's moments as soon as a node update (update_node,
-// split_update) has formed them, before the collision and the scatter.
+// Receives a node's moments as soon as a node update has formed them, before
+// the collision and the scatter.
 struct NoMomentSink {
     template <class R> __device__ __forceinline__ void operator()(const Moments<R> &) const {}
 };
@@ -1017,98 +747,375 @@ template <class T, int STRIDE> struct SharedMomentSink {
     }
 };
 
-// Half H of the update of node n (valid: n is a node); xch is the warp
-// pair's exchange area [half][moment][lane].  Both warps of a pair call it
-// once, valid or not, and pass the barrier once.
-// Returns the node's moments (those of the state it read) and plane; they
-// are meaningful for valid nodes only.
-template <int H, class S, bool SWAPPED, bool PERIODIC, class A, class Sink = NoMomentSink>
-__device__ __forceinline__ NodeOut<float> split_update(const A &a, uint32_t n, bool valid, float (&xch)[2][5][32],
-                                                       int lane, int pair, const Sink &sink = Sink()) {
-    float2 fg[Q];
-    float p[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-    Node g{};
-    int path = kNoneInside;
-    float phip = 0.f;
-    if (valid) {
-        phip = a.phip[n];   // before the barrier: half 0 overwrites it after
-        g = make_node<PERIODIC>(a, n);
-        path = node_path<PERIODIC, SWAPPED>(g);
-        if (path == kRowInside)
-            gather_half<H, S, SWAPPED, PERIODIC, kRowInside>(a, g, fg);
-        else if (SWAPPED && !PERIODIC && path == kAllInside)
-            gather_half<H, S, SWAPPED, PERIODIC, PERIODIC ? kRowInside : kAllInside>(a, g, fg);
-        else
-            gather_half<H, S, SWAPPED, PERIODIC, kNoneInside>(a, g, fg);
-        partial_moments<H>(fg, p);
-    }
-#pragma unroll
-    for (int i = 0; i < 5; i++) xch[H][i][lane] = p[i];
-    pair_barrier(pair);
-    if (!valid) return {};
-    float tot[5];
-#pragma unroll
-    for (int i = 0; i < 5; i++) tot[i] = p[i] + xch[1 - H][i][lane];
-    const float s0 = shift0(a, g);
-    Moments<float> m;
-    m.rho = tot[0];
-    m.ux = tot[1];
-    m.uy = __fadd_rn(tot[2], __fmul_rn(0.5f, __fmul_rn(a.gb, __fsub_rn(phip, a.t0))));   // as split_moments
-    m.uz = tot[3];
-    m.phi = tot[4] + s0;
-    if (a.use_phi_fix) m.phi = a.phi_fix;
-    sink(m);
-    const bool fold = SWAPPED && (path == kAllInside || (PERIODIC && path == kRowInside));
-    collide_half<H>(fg, m, a.omega_f, a.omega_g, a.force_fac, a.gb, a.t0, s0, fold ? (float)a.t_dy : 0.f);
-    if (H == 0) a.phip[n] = m.phi;
-    if (path == kRowInside)
-        scatter_half<H, S, SWAPPED, PERIODIC, kRowInside>(a, g, fg, m.rho, s0);
-    else if (SWAPPED && !PERIODIC && path == kAllInside)
-        scatter_half<H, S, SWAPPED, PERIODIC, PERIODIC ? kRowInside : kAllInside>(a, g, fg, m.rho, s0);
-    else
-        scatter_half<H, S, SWAPPED, PERIODIC, kNoneInside>(a, g, fg, m.rho, s0);
-    return {m, g.iy};
+// a - b, both lanes (the product by -1 is exact)
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return fma2(b, splat(-1.f), a); }
+// a b, both lanes, for a product that is then added: the compiler fuses a
+// paired multiplication into a paired addition, but not two scalar ones
+__device__ __forceinline__ float2 product(float2 a, float2 b) {
+    return make_float2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y));
 }
 
-// The moments of node g exactly as step16_split_kernel's two halves form
-// them (the same loads on the same path, the same partial sums, added in the
-// same order), so observables reduced from them match those the kernel
-// reduces when it steps (the observables of its OBS variant).
-template <class S, bool SWAPPED, bool PERIODIC, class A>
-__device__ __forceinline__ Moments<float> split_moments(const A &a, const Node &g) {
-    float2 fg[Q];
+// Where the g values of a 16-bit node are re-referenced from plane to plane
+// (read_shift_delta, write_shift_delta).  BGK folds it into its relaxation
+// where every neighbour is inside: on the rows of a periodic box, and in a
+// closed box for warps without an x-wall node (fold = t_dy, per-value
+// spacing 0); elsewhere it is added value by value (fold 0, spacing t_dy).
+struct Shift {
+    float s0;     // the node's own T_c
+    float t_dy;   // plane spacing applied value by value
+    float fold;   // plane spacing folded into the relaxation
+};
+
+// Population K's re-referencing on reading, and I's on writing, for a plane
+// spacing t_dy.
+template <bool SWAPPED, int K, int INTERIOR> __device__ __forceinline__ float read_shift(const Node &g, float t_dy) {
+    if constexpr (!SWAPPED || cy(K) == 0) return 0.f;
+    else return inside_t<INTERIOR, -cx(K), -cy(K), -cz(K)>(g) ? (float)cy(K) * t_dy : 0.f;
+}
+template <bool SWAPPED, int I, int INTERIOR> __device__ __forceinline__ float write_shift(const Node &g, float t_dy) {
+    if constexpr (!SWAPPED || cy(I) == 0) return 0.f;
+    else return inside_t<INTERIOR, cx(I), cy(I), cz(I)>(g) ? (float)cy(I) * t_dy : 0.f;
+}
+
+// Whether population I of node g leaves through a plate with the
+// anti-bounce-back rule (and not also through a z wall, see the top).
+template <bool PERIODIC, int INTERIOR, int I> __device__ __forceinline__ bool meets_plate(const Node &g) {
+    if constexpr (INTERIOR != kNoneInside || cy(I) == 0) return false;
+    else
+        return (cy(I) < 0 ? !g.vym : !g.vyp) &&
+               !(!PERIODIC && ((cz(I) < 0 && !g.vzm) || (cz(I) > 0 && !g.vzp)));
+}
+
+// Stores the word of population I of node g where the next step reads it.
+template <class S, bool SWAPPED, bool PERIODIC, int INTERIOR, int I, class A>
+__device__ __forceinline__ void store_word(const A &a, const Node &g, typename Pack16<S>::T w) {
+    constexpr int DX = cx(I), DY = cy(I), DZ = cz(I);
+    const bool in = SWAPPED && inside_t<INTERIOR, DX, DY, DZ>(g);
+    if constexpr (selects_address<SWAPPED, PERIODIC, INTERIOR, I>())
+        *(in ? a.st2(I, (int32_t)g.n + disp<DX, DY, DZ>(g)) : a.st2(opp(I), g.n)) = w;
+    else if (in)
+        *a.st2(I, (int32_t)g.n + disp<DX, DY, DZ>(g)) = w;
+    else
+        *a.st2(opp(I), g.n) = w;
+}
+
+// ---- BGK ----
+//
+// collide_fast in the normalised variables:
+//   fh*_i = fh_i - (fh_i - (rho + p_i)) / tau + 3 (1 - 1/(2 tau)) F_y (c_iy - u_y) (1 + p_i)
+//   gh*_i = gh_i - (gh_i + s0 - phi (1 + p_i)) / tau_c,
+// p_i = 3 c_i.u + 4.5 (c_i.u)^2 - 1.5 u^2: no weight on load or store.
+// B200, 256^3 FP16S, periodic: 582 us per step in the natural layout and 626
+// in the swapped one, against 664 and 652 with a node's update split over
+// two warps that exchanged their partial moments through shared memory (64
+// registers, 770-820 instructions per 32 nodes and a barrier; here ~550, no
+// barrier, and 27 loads in flight per warp instead of 13).  Closed box: 609
+// and 711 against 674 and 710.
+
+// The half of the opposite pairs that population k is summed in.  The
+// moments are two partial sums, added: the rest population and the pairs of
+// 1, 2, 5, 7, 19 and 20, and the other seven pairs.
+__host__ __device__ constexpr int pair_rep(int k) { return k < opp(k) ? k : opp(k); }
+__host__ __device__ constexpr int half_of(int k) {
+    return (k == 0 || pair_rep(k) == 1 || pair_rep(k) == 2 || pair_rep(k) == 5 || pair_rep(k) == 7 ||
+            pair_rep(k) == 19 || pair_rep(k) == 20)
+               ? 0
+               : 1;
+}
+
+// Half H's share of rho, j_x, j_y, j_z and sum w_i gh_i: sums per weight
+// class, then weighted; f and g paired.
+template <int H, class Value> __device__ __forceinline__ void half_sums(const Value &value, float (&p)[5]) {
+    float2 rt[4] = {};   // (sum fh, sum gh) per weight class
+    float x[4] = {0.f, 0.f, 0.f, 0.f}, y[4] = {0.f, 0.f, 0.f, 0.f}, z[4] = {0.f, 0.f, 0.f, 0.f};
+    Unroll<0, Q>::run([&](auto kk) {
+        constexpr int K = decltype(kk)::value;
+        if constexpr (half_of(K) == H) {
+            constexpr int C = wclass(K);
+            const float2 v = value(kk);
+            rt[C] = add2(rt[C], v);
+            if (cx(K) > 0) x[C] += v.x;
+            if (cx(K) < 0) x[C] -= v.x;
+            if (cy(K) > 0) y[C] += v.x;
+            if (cy(K) < 0) y[C] -= v.x;
+            if (cz(K) > 0) z[C] += v.x;
+            if (cz(K) < 0) z[C] -= v.x;
+        }
+    });
+    const float w0 = (float)wd(0), w1 = (float)wd(1), w2 = (float)wd(7), w3 = (float)wd(19);
+    const float2 s = fma2(splat(w3), rt[3], fma2(splat(w2), rt[2], fma2(splat(w1), rt[1], mul2(splat(w0), rt[0]))));
+    p[0] = s.x;
+    p[1] = fmaf(w3, x[3], fmaf(w2, x[2], w1 * x[1]));
+    p[2] = fmaf(w3, y[3], fmaf(w2, y[2], w1 * y[1]));
+    p[3] = fmaf(w3, z[3], fmaf(w2, z[2], w1 * z[1]));
+    p[4] = s.y;
+}
+
+template <class A, class Value>
+__device__ __forceinline__ Moments<float> bgk_moments(const A &a, const Value &value, float phip, float s0) {
     float p0[5], p1[5];
-    const int path = node_path<PERIODIC, SWAPPED>(g);
-    if (path == kRowInside) {
-        gather_half<0, S, SWAPPED, PERIODIC, kRowInside>(a, g, fg);
-        gather_half<1, S, SWAPPED, PERIODIC, kRowInside>(a, g, fg);
-    } else if (SWAPPED && !PERIODIC && path == kAllInside) {
-        gather_half<0, S, SWAPPED, PERIODIC, PERIODIC ? kRowInside : kAllInside>(a, g, fg);
-        gather_half<1, S, SWAPPED, PERIODIC, PERIODIC ? kRowInside : kAllInside>(a, g, fg);
-    } else {
-        gather_half<0, S, SWAPPED, PERIODIC, kNoneInside>(a, g, fg);
-        gather_half<1, S, SWAPPED, PERIODIC, kNoneInside>(a, g, fg);
-    }
-    partial_moments<0>(fg, p0);
-    partial_moments<1>(fg, p1);
+    half_sums<0>(value, p0);
+    half_sums<1>(value, p1);
     Moments<float> m;
     m.rho = p0[0] + p1[0];
     m.ux = p0[1] + p1[1];
-    m.uy = __fadd_rn(p0[2] + p1[2], __fmul_rn(0.5f, __fmul_rn(a.gb, __fsub_rn((float)a.phip[g.n], a.t0))));
+    m.uy = __fadd_rn(p0[2] + p1[2], __fmul_rn(0.5f, __fmul_rn(a.gb, __fsub_rn(phip, a.t0))));
     m.uz = p0[3] + p1[3];
-    m.phi = (p0[4] + p1[4]) + shift0(a, g);
+    m.phi = (p0[4] + p1[4]) + s0;   // sum w_i (gh_i + s0)
     if (a.use_phi_fix) m.phi = a.phi_fix;
     return m;
+}
+
+// Both relaxations are affine maps of the old value, with per-node
+// coefficients (k = kf (c_y - u_y) takes three values, one per c_y):
+//   fh* = (1 - om_f) fh + (om_f rho + k) + (om_f + k) p
+//   gh* = (1 - om_g) gh + om_g (phi - s0) + om_g phi p
+// and p_I, p_J = (q +/- 2 eu) / 2 with q = eu^2 - 3 u^2: two paired
+// multiply-adds per population and three per pair.  With the folded shift:
+// ag (v + c_y fold) + ... + c_y fold = ag v + ... + (ag + 1) c_y fold.
+template <class S, bool SWAPPED, bool PERIODIC, int INTERIOR, class A, class Value>
+__device__ __forceinline__ void bgk_relax_store(const A &a, const Node &g, const Value &value,
+                                                const Moments<float> &m, const Shift &sh) {
+    const float om_f = a.omega_f, om_g = a.omega_g, s0 = sh.s0;
+    const float ux3 = 3.f * m.ux, uy3 = 3.f * m.uy, uz3 = 3.f * m.uz;
+    const float uv = 3.f * (m.ux * m.ux + m.uy * m.uy + m.uz * m.uz);
+    const float kf = 3.f * a.force_fac * (a.gb * (m.phi - a.t0));
+    const float k_m = kf * (-1.f - m.uy), k_0 = kf * (-m.uy), k_p = kf * (1.f - m.uy);
+    const float af = 1.f - om_f, orho = om_f * m.rho;
+    const float c0[3] = {orho + k_m, orho + k_0, orho + k_p};   // indexed by c_y + 1
+    const float c1[3] = {om_f + k_m, om_f + k_0, om_f + k_p};
+    const float ag = 1.f - om_g, d1 = om_g * m.phi, d0 = om_g * (m.phi - s0);
+    const float df = (ag + 1.f) * sh.fold;
+    const float d0c[3] = {d0 - df, d0, d0 + df};
+    const float2 a2 = make_float2(af, ag);
+    // (fh, gh) <- (af fh + c1 p + c0, ag gh + d1 p + d0c): both at once
+    auto relax = [&](auto kk, float p) {
+        constexpr int K = decltype(kk)::value, Y = cy(K) + 1;
+        const float2 v = fma2(a2, value(kk), fma2(make_float2(c1[Y], d1), splat(p), make_float2(c0[Y], d0c[Y])));
+        float gv = v.y;
+        if (meets_plate<PERIODIC, INTERIOR, K>(g))
+            gv = 2.f * (cy(K) < 0 ? a.t_hot : a.t_cold) * (1.f + m.rho) - gv - 2.f * s0;
+        if constexpr (!(SWAPPED && all_inside<INTERIOR, PERIODIC>())) gv += write_shift<SWAPPED, K, INTERIOR>(g, sh.t_dy);
+        store_word<S, SWAPPED, PERIODIC, INTERIOR, K>(a, g, Pack16<S>::pack(v.x, gv));
+    };
+    relax(std::integral_constant<int, 0>{}, -0.5f * uv);
+    // corners, edges, faces: of the orders tried, the one whose registers
+    // spill least where it costs (closed box, swapped layout: 706 us at 256^3
+    // FP16S and 150 at 192x96x192 BF16S, against 709 and 169 in index order)
+    auto pairs = [&](auto cls) {
+        Unroll<1, Q>::run([&](auto ii) {
+            constexpr int I = decltype(ii)::value;
+            constexpr int J = opp(I);
+            if constexpr (I < J && wclass(I) == decltype(cls)::value) {
+                float eu = 0.f;
+                if (cx(I) > 0) eu += ux3;
+                if (cx(I) < 0) eu -= ux3;
+                if (cy(I) > 0) eu += uy3;
+                if (cy(I) < 0) eu -= uy3;
+                if (cz(I) > 0) eu += uz3;
+                if (cz(I) < 0) eu -= uz3;
+                const float q = fmaf(eu, eu, -uv);
+                relax(ii, fmaf(0.5f, q, eu));
+                relax(std::integral_constant<int, J>{}, fmaf(0.5f, q, -eu));
+            }
+        });
+    };
+    pairs(std::integral_constant<int, 3>{});
+    pairs(std::integral_constant<int, 2>{});
+    pairs(std::integral_constant<int, 1>{});
+}
+
+// ---- regularised collision ----
+//
+// collide_reg, operation for operation (each an explicit round-to-nearest
+// one, so the single-case and the batch kernels give bitwise the same
+// state).  What leaves the collision depends on the old populations only
+// through 18 sums, so a population is dead once it is summed, and opposite
+// directions share c.u, c.j and q; the sums of f and g and the two
+// directions of a pair go two to an instruction.  B200, 256^3 FP16S, per
+// step: 654 us periodic, 719 closed box, against 1157 and 1186 with all 54
+// values held unpacked (128 registers, 16 warps per SM, ~1600 instructions).
+struct RegSums {
+    Moments<float> m;
+    float sxx, syy, szz, sxy, sxz, syz;   // second moments of f
+    float jx, jy, jz;                     // first moments of g
+};
+
+// value(K): (f_K, g_K)
+template <class A, class Value>
+__device__ __forceinline__ RegSums reg_sums(const A &a, const Value &value, float phip) {
+    float2 r = {}, jx = {}, jy = {}, jz = {};   // of (f, g)
+    RegSums t = {};
+    Unroll<0, Q>::run([&](auto kk) {
+        constexpr int K = decltype(kk)::value;
+        constexpr int X = cx(K), Y = cy(K), Z = cz(K);
+        const float2 v = value(kk);
+        r = add2(r, v);
+        if (X != 0) jx = X > 0 ? add2(jx, v) : sub2(jx, v);
+        if (Y != 0) jy = Y > 0 ? add2(jy, v) : sub2(jy, v);
+        if (Z != 0) jz = Z > 0 ? add2(jz, v) : sub2(jz, v);
+        if (X != 0) t.sxx = add_rn(t.sxx, v.x);
+        if (Y != 0) t.syy = add_rn(t.syy, v.x);
+        if (Z != 0) t.szz = add_rn(t.szz, v.x);
+        if (X * Y != 0) t.sxy = X * Y > 0 ? add_rn(t.sxy, v.x) : sub_rn(t.sxy, v.x);
+        if (X * Z != 0) t.sxz = X * Z > 0 ? add_rn(t.sxz, v.x) : sub_rn(t.sxz, v.x);
+        if (Y * Z != 0) t.syz = Y * Z > 0 ? add_rn(t.syz, v.x) : sub_rn(t.syz, v.x);
+    });
+    t.m.rho = r.x;
+    t.m.ux = jx.x;
+    t.m.uy = add_rn(jy.x, mul_rn(0.5f, mul_rn(a.gb, sub_rn(phip, a.t0))));
+    t.m.uz = jz.x;
+    t.m.phi = r.y;
+    if (a.use_phi_fix) t.m.phi = a.phi_fix;
+    t.jx = jx.y;
+    t.jy = jy.y;
+    t.jz = jz.y;
+    return t;
+}
+
+template <class S, bool SWAPPED, bool PERIODIC, int INTERIOR, class A>
+__device__ __forceinline__ void reg_relax_store(const A &a, const Node &g, const RegSums &t, const Shift &sh) {
+    const Moments<float> &m = t.m;
+    const float third = 1.f / 3.f;
+    const float rho3 = mul_rn(m.rho, third);
+    const float pxx = fma_rn(-m.ux, m.ux, sub_rn(t.sxx, rho3));
+    const float pyy = fma_rn(-m.uy, m.uy, sub_rn(t.syy, rho3));
+    const float pzz = fma_rn(-m.uz, m.uz, sub_rn(t.szz, rho3));
+    const float pxy2 = mul_rn(2.f, fma_rn(-m.ux, m.uy, t.sxy));
+    const float pxz2 = mul_rn(2.f, fma_rn(-m.ux, m.uz, t.sxz));
+    const float pyz2 = mul_rn(2.f, fma_rn(-m.uy, m.uz, t.syz));
+    const float tr3 = mul_rn(add_rn(add_rn(pxx, pyy), pzz), third);
+    const float jx = fma_rn(-m.phi, m.ux, t.jx), jy = fma_rn(-m.phi, m.uy, t.jy), jz = fma_rn(-m.phi, m.uz, t.jz);
+    const float keep_f = mul_rn(4.5f, sub_rn(1.f, a.omega_f)), keep_g = mul_rn(3.f, sub_rn(1.f, a.omega_g));
+    const float uv = mul_rn(3.f, fma_rn(m.uz, m.uz, fma_rn(m.uy, m.uy, mul_rn(m.ux, m.ux))));
+    const float kf = mul_rn(mul_rn(3.f, a.force_fac), mul_rn(a.gb, sub_rn(m.phi, a.t0)));
+    const float k[3] = {mul_rn(kf, sub_rn(-1.f, m.uy)), mul_rn(kf, sub_rn(0.f, m.uy)), mul_rn(kf, sub_rn(1.f, m.uy))};
+    // population K's value out, normalised and relative to T_c where it goes
+    auto put = [&](auto kk, float fv, float gv) {
+        constexpr int K = decltype(kk)::value;
+        if (meets_plate<PERIODIC, INTERIOR, K>(g)) gv = abb<K>(gv, cy(K) < 0 ? a.t_hot : a.t_cold, m.rho);
+        const float sl = sub_rn(sh.s0, write_shift<SWAPPED, K, INTERIOR>(g, sh.t_dy));
+        store_word<S, SWAPPED, PERIODIC, INTERIOR, K>(
+            a, g, Pack16<S>::pack(mul_rn(fv, (float)winv(K)), fma_rn(gv, (float)winv(K), -sl)));
+    };
+    {   // the rest population
+        const float w = (float)wd(0);
+        const float p = add_rn(0.f, mul_rn(0.5f, -uv));
+        const float feq0 = mul_rn(w, add_rn(1.f, p));
+        const float fneq = mul_rn(mul_rn(keep_f, w), -tr3);
+        const float fv = add_rn(add_rn(mul_rn(w, add_rn(m.rho, p)), fneq), mul_rn(k[1], feq0));
+        put(std::integral_constant<int, 0>{}, fv, mul_rn(m.phi, feq0));
+    }
+    Unroll<1, Q>::run([&](auto ii) {
+        constexpr int I = decltype(ii)::value;
+        constexpr int J = opp(I);
+        constexpr int X = cx(I), Y = cy(I), Z = cz(I);
+        if constexpr (I < J) {
+            // c.u, c.j in the order x, y, z (of J: the negatives); q of both
+            auto dot = [](float x, float y, float z) {
+                float d = X > 0 ? x : -x;
+                if constexpr (Y != 0) d = X != 0 ? (Y > 0 ? add_rn(d, y) : sub_rn(d, y)) : Y > 0 ? y : -y;
+                if constexpr (Z != 0) d = X != 0 || Y != 0 ? (Z > 0 ? add_rn(d, z) : sub_rn(d, z)) : Z > 0 ? z : -z;
+                return d;
+            };
+            const float w = (float)wd(I);
+            const float eu = mul_rn(3.f, dot(m.ux, m.uy, m.uz)), cj = dot(jx, jy, jz);
+            float q = -tr3;
+            if (X != 0) q = add_rn(q, pxx);
+            if (Y != 0) q = add_rn(q, pyy);
+            if (Z != 0) q = add_rn(q, pzz);
+            if (X * Y != 0) q = X * Y > 0 ? add_rn(q, pxy2) : sub_rn(q, pxy2);
+            if (X * Z != 0) q = X * Z > 0 ? add_rn(q, pxz2) : sub_rn(q, pxz2);
+            if (Y * Z != 0) q = Y * Z > 0 ? add_rn(q, pyz2) : sub_rn(q, pyz2);
+            // lanes: I, J
+            const float2 p = add2(make_float2(eu, -eu), splat(mul_rn(0.5f, fma_rn(eu, eu, -uv))));
+            const float2 feq0 = mul2(splat(w), add2(splat(1.f), p));
+            const float2 force = product(make_float2(k[1 + Y], k[1 - Y]), feq0);
+            const float2 feq = product(splat(w), add2(splat(m.rho), p));
+            const float2 fv = add2(add2(feq, splat(mul_rn(mul_rn(keep_f, w), q))), force);
+            const float2 gv = fma2(splat(mul_rn(keep_g, w)), make_float2(cj, -cj), mul2(splat(m.phi), feq0));
+            put(ii, fv.x, gv.x);
+            put(std::integral_constant<int, J>{}, fv.y, gv.y);
+        }
+    });
+}
+
+// ---- one node ----
+
+// Moments of node g on the path INTERIOR, then (with STORE) its collision and
+// its stores.  all_in: whether the warp's lanes on this path have all their
+// neighbours inside (a closed box's rows; see Shift).
+template <class S, bool SWAPPED, bool PERIODIC, int COLL, int INTERIOR, bool STORE, class A, class Sink>
+__device__ __forceinline__ Moments<float> update_path16(const A &a, const Node &g, bool all_in, const Sink &sink) {
+    const float phip = a.phip[g.n];
+    const bool folded = COLL == LBM_COLLISION_BGK && SWAPPED && (all_inside<INTERIOR, PERIODIC>() || all_in);
+    const Shift sh = {shift0(a, g), folded ? 0.f : (float)a.t_dy, folded ? (float)a.t_dy : 0.f};
+    typename Pack16<S>::T w[Q];
+    Unroll<0, Q>::run([&](auto kk) {
+        constexpr int K = decltype(kk)::value;
+        w[K] = load_pair<S, SWAPPED, PERIODIC, K, INTERIOR>(a, g);
+    });
+    if constexpr (COLL == LBM_COLLISION_REGULARIZED) {
+        auto value = [&](auto kk) {   // w_K (fh, gh + T_c at the location)
+            constexpr int K = decltype(kk)::value;
+            const float2 v = Pack16<S>::unpack(w[K]);
+            const float at = add_rn(sh.s0, read_shift<SWAPPED, K, INTERIOR>(g, sh.t_dy));
+            return product(splat((float)wd(K)), make_float2(v.x, add_rn(v.y, at)));
+        };
+        const RegSums t = reg_sums(a, value, phip);
+        if constexpr (STORE) {
+            sink(t.m);
+            const Node gs = again(a, g);
+            a.phip[gs.n] = t.m.phi;
+            reg_relax_store<S, SWAPPED, PERIODIC, INTERIOR>(a, gs, t, sh);
+        }
+        return t.m;
+    } else {
+        auto value = [&](auto kk) {   // gh relative to the node's T_c (folded: as stored)
+            constexpr int K = decltype(kk)::value;
+            float2 v = Pack16<S>::unpack(w[K]);
+            if constexpr (!(SWAPPED && all_inside<INTERIOR, PERIODIC>())) v.y += read_shift<SWAPPED, K, INTERIOR>(g, sh.t_dy);
+            return v;
+        };
+        const Moments<float> m = bgk_moments(a, value, phip, sh.s0);
+        if constexpr (STORE) {
+            sink(m);
+            const Node gs = again(a, g);
+            a.phip[gs.n] = m.phi;
+            bgk_relax_store<S, SWAPPED, PERIODIC, INTERIOR>(a, gs, value, m, sh);
+        }
+        return m;
+    }
+}
+
+// Two bodies only, and nothing but the node crosses the branch.  A closed
+// box's rows take one body whether or not a warp holds an x-wall node, with
+// the x-moving addresses by a select: a third body for the warps without one
+// saves its warps the selects but competes for the instruction cache (B200,
+// closed-box swapped step, BGK: 701 us at 256^3 FP16S with two bodies, 717
+// with three; 152 against 162 at 192x96x192 BF16S).
+template <class S, bool SWAPPED, bool PERIODIC, int COLL, bool STORE, class A, class Sink>
+__device__ __forceinline__ Moments<float> update_node16(const A &a, const Node &g, const Sink &sink) {
+    const int path = node_path<PERIODIC, SWAPPED>(g);
+    if (path != kNoneInside)
+        return update_path16<S, SWAPPED, PERIODIC, COLL, kRowInside, STORE>(a, g, path == kAllInside, sink);
+    return update_path16<S, SWAPPED, PERIODIC, COLL, kNoneInside, STORE>(a, g, false, sink);
+}
+
+// The moments of node g exactly as the 16-bit step forms them, so observables
+// reduced from them match those an observed step reduces.
+template <class S, bool SWAPPED, bool PERIODIC, int COLL, class A>
+__device__ __forceinline__ Moments<float> step_moments16(const A &a, const Node &g) {
+    return update_node16<S, SWAPPED, PERIODIC, COLL, false>(a, g, NoMomentSink{});
 }
 
 template <class S, bool SWAPPED, bool PERIODIC, int COLL = LBM_COLLISION_BGK, class A, class Sink = NoMomentSink>
 __device__ __forceinline__ NodeOut<typename Codec<S>::R> update_node(const A &a, uint32_t n,
                                                                      const Sink &sink = Sink()) {
-    if constexpr (sizeof(S) == 2 && COLL == LBM_COLLISION_BGK) {
-        const auto o = update_node_norm<S, SWAPPED, PERIODIC>(a, n);
-        sink(o.m);
-        return o;
-    }
+    if constexpr (sizeof(S) == 2) {
+        const Node g = make_node<PERIODIC>(a, n);
+        return {update_node16<S, SWAPPED, PERIODIC, COLL, true>(a, g, sink), g.iy};
+    } else {
     using R = typename Codec<S>::R;
     const Node g = make_node<PERIODIC>(a, n);
     R fr[Q], gr[Q];
@@ -1144,6 +1151,7 @@ __device__ __forceinline__ NodeOut<typename Codec<S>::R> update_node(const A &a,
     else
         scatter<S, SWAPPED, PERIODIC, kNoneInside>(a, g, fr, gr, m.rho);
     return {m, g.iy};
+    }
 }
 
 // One time step.  With OBS, the kernel also reduces the observables of the
@@ -1151,22 +1159,25 @@ __device__ __forceinline__ NodeOut<typename Codec<S>::R> update_node(const A &a,
 // row of kObsTerms FP64 sums per warp (a.obs_rows, row W b + w for warp w of
 // block b, W = node_threads / 32), at no extra read of the populations.
 template <class S, bool SWAPPED, bool PERIODIC, int COLL, bool OBS = false>
-__global__ void __launch_bounds__(128, StepOccupancy<S>::value) step_kernel(const StepArgs<S> a) {
+__global__ void __launch_bounds__(bound_threads<S>(), step_threads_per_sm<S>() / bound_threads<S>())
+    step_kernel(const StepArgs<S> a) {
     const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
     if constexpr (!OBS) {
         if (n >= a.nodes) return;
         update_node<S, SWAPPED, PERIODIC, COLL>(a, n);
     } else {
-        __shared__ double parked[5][128];   // ux, uy, uz, phi, rho per thread
+        using T = typename Codec<S>::R;
+        constexpr int kT = node_threads<S>();
+        __shared__ T parked[5][kT];   // ux, uy, uz, phi, rho per thread
         // the terms of add_obs_terms: uy*phi, |u|^2, ux, uy, uz, phi
         double d[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
         int iy = 0;
         bool bad = false;
         const bool valid = n < a.nodes;
         if (valid) {
-            volatile double *mine = &parked[0][threadIdx.x];
-            iy = update_node<S, SWAPPED, PERIODIC, COLL>(a, n, SharedMomentSink<double, 128>{mine}).iy;
-            const double ux = mine[0], uy = mine[128], uz = mine[256], phi = mine[384], rho = mine[512];
+            volatile T *mine = &parked[0][threadIdx.x];
+            iy = update_node<S, SWAPPED, PERIODIC, COLL>(a, n, SharedMomentSink<T, kT>{mine}).iy;
+            const double ux = mine[0], uy = mine[kT], uz = mine[2 * kT], phi = mine[3 * kT], rho = mine[4 * kT];
             d[0] = uy * phi;
             d[1] = ux * ux + uy * uy + uz * uz;
             d[2] = ux;
@@ -1177,56 +1188,6 @@ __global__ void __launch_bounds__(128, StepOccupancy<S>::value) step_kernel(cons
         }
         const size_t warp_row = (size_t)blockIdx.x * (node_threads<S>() / 32) + (threadIdx.x >> 5);
         warp_obs_row(d, iy, valid, bad, a.ly, a.obs_rows + warp_row * kObsTerms);
-    }
-}
-
-// 16-bit storage, BGK: block b updates nodes [64 b, 64 b + 64); warps 2p
-// and 2p + 1 share nodes 64 b + 32 p + lane (split_update).  8 blocks of
-// 128 threads per SM (64 registers, no spills): B200, 256^3, 24.6 GLUPS
-// FP16S and 23.7 BF16S, against 20.7 and 21.3 for the one-thread-per-node
-// kernel at 4 blocks.
-//
-// With OBS, the kernel also reduces the observables of the state it reads
-// into one row of kObsTerms FP64 sums per warp pair (a.obs_rows, row 2 b + p
-// for pair p of block b): half 0 parks its 32 nodes' moments in shared memory
-// when it forms them and reduces them after its update; half 1 leaves when
-// its update is done.  (Splitting the reduction between the halves measured
-// slower: both then form the terms.)
-constexpr int kSplitBlocks = 8;
-template <class S, bool SWAPPED, bool PERIODIC, bool OBS = false>
-__global__ void __launch_bounds__(128, kSplitBlocks) step16_split_kernel(const StepArgs<S> a) {
-    __shared__ float xch[2][2][5][32];   // [warp pair][half][moment][lane]
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int pair = warp >> 1;
-    const uint32_t n = blockIdx.x * 64u + (uint32_t)(pair * 32 + lane);
-    const bool valid = n < a.nodes;
-    if constexpr (!OBS) {
-        if ((warp & 1) == 0)
-            split_update<0, S, SWAPPED, PERIODIC>(a, n, valid, xch[pair], lane, pair);
-        else
-            split_update<1, S, SWAPPED, PERIODIC>(a, n, valid, xch[pair], lane, pair);
-    } else {
-        __shared__ float parked[2][5][32];   // [warp pair][ux, uy, uz, phi, rho][lane]
-        if (warp & 1) {
-            split_update<1, S, SWAPPED, PERIODIC>(a, n, valid, xch[pair], lane, pair);
-            return;
-        }
-        volatile float *mine = &parked[pair][0][lane];
-        const int iy = split_update<0, S, SWAPPED, PERIODIC>(a, n, valid, xch[pair], lane, pair,
-                                                             SharedMomentSink<float, 32>{mine}).iy;
-        double d[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-        bool bad = false;
-        if (valid) {
-            const double ux = mine[0], uy = mine[32], uz = mine[64], phi = mine[96], rho = mine[128];
-            d[0] = uy * phi;
-            d[1] = ux * ux + uy * uy + uz * uz;
-            d[2] = ux;
-            d[3] = uy;
-            d[4] = uz;
-            d[5] = phi;
-            bad = !isfinite(ux) || !isfinite(uy) || !isfinite(uz) || !isfinite(phi) || !isfinite(rho);
-        }
-        warp_obs_row(d, iy, valid, bad, a.ly, a.obs_rows + ((size_t)blockIdx.x * 2 + pair) * kObsTerms);
     }
 }
 
