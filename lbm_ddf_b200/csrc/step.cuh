@@ -178,19 +178,12 @@ __device__ __forceinline__ bool inside(const Node &g) {
 //                at the x walls of a closed box;
 //   kAllInside:  all of them (a closed box's rows whose warp holds no x-wall
 //                node: with LX a multiple of 32, all but the first and last
-//                warp of a row);
-//   kRowLoWall, kRowHiWall: as kRowInside, in a closed box's warp whose
-//                x-wall nodes, if any, all lie at x = 0 (Lo) or all at
-//                x = LX-1 (Hi): only the x neighbour on that side is tested
-//                (the first and last warp of a row, with LX a multiple of 32
-//                and at least 64).
-constexpr int kNoneInside = 0, kRowInside = 1, kAllInside = 2, kRowLoWall = 3, kRowHiWall = 4;
+//                warp of a row).
+constexpr int kNoneInside = 0, kRowInside = 1, kAllInside = 2;
 template <int INTERIOR, int DX, int DY, int DZ>
 __device__ __forceinline__ bool inside_t(const Node &g) {
     if constexpr (INTERIOR == kAllInside) return true;
     else if constexpr (INTERIOR == kRowInside) return DX < 0 ? g.vxm : DX > 0 ? g.vxp : true;
-    else if constexpr (INTERIOR == kRowLoWall) return DX < 0 ? g.vxm : true;
-    else if constexpr (INTERIOR == kRowHiWall) return DX > 0 ? g.vxp : true;
     else return inside<DX, DY, DZ>(g);
 }
 // whether every neighbour of a node taking this path is inside (so the
@@ -221,21 +214,6 @@ template <bool PERIODIC, bool SWAPPED = true> __device__ __forceinline__ int nod
     }
     return kRowInside;
 }
-// node_path, with a closed box's warps at one x wall told apart (kRowLoWall,
-// kRowHiWall), for the FP32 and FP64 updates of the swapped layout.
-template <bool PERIODIC> __device__ __forceinline__ int node_path_x(const Node &g) {
-    if (!yz_interior<PERIODIC>(g)) return kNoneInside;
-    if constexpr (!PERIODIC) {
-        const unsigned active = __activemask();
-        const bool lo_in = __all_sync(active, g.vxm), hi_in = __all_sync(active, g.vxp);
-        if (lo_in && hi_in) return kAllInside;
-        if (hi_in) return kRowLoWall;
-        if (lo_in) return kRowHiWall;
-        return kNoneInside;   // a warp at both x walls (rows shorter than 64 or not whole warps)
-    }
-    return kRowInside;
-}
-
 // Population k (of f when WHICH = 0, of g when 1) of node g at the current
 // time, from either layout.  `a` supplies the addresses: a.ldp(which, k,
 // node).  In the swapped layout the value sits at the neighbour x - c_K
@@ -568,30 +546,38 @@ __device__ __forceinline__ R abb(R gv, R tw, R rho) {
         return -gv + R(2) * R(wd(I)) * tw * (R(1) + rho);
 }
 
-// Write the post-collision populations of node g to where the next step
-// reads them.  rho is the node's pre-collision density (for anti-bounce-back).
+// Whether population I of node g leaves through a plate with the
+// anti-bounce-back rule (and not also through a z wall, see the top).
+template <bool PERIODIC, int INTERIOR, int I> __device__ __forceinline__ bool meets_plate(const Node &g) {
+    if constexpr (INTERIOR != kNoneInside || cy(I) == 0) return false;
+    else
+        return (cy(I) < 0 ? !g.vym : !g.vyp) &&
+               !(!PERIODIC && ((cz(I) < 0 && !g.vzm) || (cz(I) > 0 && !g.vzp)));
+}
+
+// Stores population I (of f when which = 0, of g when 1) of node g where the
+// next step reads it: the neighbour x + c_I (swapped layout, inside) or the
+// node itself, the address chosen by a select (see load_pop).
+template <bool SWAPPED, int INTERIOR, int I, class A, class R>
+__device__ __forceinline__ void store_pop(const A &a, const Node &g, int which, R v) {
+    constexpr int DX = cx(I), DY = cy(I), DZ = cz(I);
+    const bool in = SWAPPED && inside_t<INTERIOR, DX, DY, DZ>(g);
+    *(in ? &a.st(which, I, (int32_t)g.n + disp<DX, DY, DZ>(g)) : &a.st(which, opp(I), g.n)) = v;
+}
+
+// Writes the post-collision populations of node g to where the next step
+// reads them (FP32 and FP64).  rho is the node's pre-collision density (for
+// anti-bounce-back).
 template <class S, bool SWAPPED, bool PERIODIC, int INTERIOR = kNoneInside, class A>
 __device__ __forceinline__ void scatter(const A &a, const Node &g, const typename Codec<S>::R (&fr)[Q],
                                         const typename Codec<S>::R (&gr)[Q], typename Codec<S>::R rho) {
-    using C = Codec<S>;
-    using R = typename C::R;
+    static_assert(elem_stride<S>() == 1, "16-bit pairs are stored by store_word");
     Unroll<0, Q>::run([&](auto ii) {
         constexpr int I = decltype(ii)::value;
-        constexpr int DX = cx(I), DY = cy(I), DZ = cz(I);
-        R fv = fr[I];
-        R gv = gr[I];
-        const bool out_y = INTERIOR == kNoneInside && ((DY < 0 && !g.vym) || (DY > 0 && !g.vyp));
-        const bool out_z = !PERIODIC && INTERIOR == kNoneInside && ((DZ < 0 && !g.vzm) || (DZ > 0 && !g.vzp));
-        if (DY != 0 && out_y && !out_z) gv = abb<I>(gv, DY < 0 ? a.t_hot : a.t_cold, rho);
-        static_assert(elem_stride<S>() == 1, "16-bit pairs are stored by put_pair");
-        {
-            // to the neighbour x + c_I (swapped layout, inside) or back to
-            // the node itself, the address chosen by a select (see load_pop)
-            const bool in = SWAPPED && inside_t<INTERIOR, DX, DY, DZ>(g);
-            const int32_t j = (int32_t)g.n + disp<DX, DY, DZ>(g);
-            *(in ? &a.st(0, I, j) : &a.st(0, opp(I), g.n)) = C::template f_out<I>(fv, a.t0);
-            *(in ? &a.st(1, I, j) : &a.st(1, opp(I), g.n)) = C::template g_out<I>(gv, a.t0);
-        }
+        typename Codec<S>::R gv = gr[I];
+        if (meets_plate<PERIODIC, INTERIOR, I>(g)) gv = abb<I>(gv, cy(I) < 0 ? a.t_hot : a.t_cold, rho);
+        store_pop<SWAPPED, INTERIOR, I>(a, g, 0, fr[I]);
+        store_pop<SWAPPED, INTERIOR, I>(a, g, 1, gv);
     });
 }
 
@@ -775,15 +761,6 @@ template <bool SWAPPED, int K, int INTERIOR> __device__ __forceinline__ float re
 template <bool SWAPPED, int I, int INTERIOR> __device__ __forceinline__ float write_shift(const Node &g, float t_dy) {
     if constexpr (!SWAPPED || cy(I) == 0) return 0.f;
     else return inside_t<INTERIOR, cx(I), cy(I), cz(I)>(g) ? (float)cy(I) * t_dy : 0.f;
-}
-
-// Whether population I of node g leaves through a plate with the
-// anti-bounce-back rule (and not also through a z wall, see the top).
-template <bool PERIODIC, int INTERIOR, int I> __device__ __forceinline__ bool meets_plate(const Node &g) {
-    if constexpr (INTERIOR != kNoneInside || cy(I) == 0) return false;
-    else
-        return (cy(I) < 0 ? !g.vym : !g.vyp) &&
-               !(!PERIODIC && ((cz(I) < 0 && !g.vzm) || (cz(I) > 0 && !g.vzp)));
 }
 
 // Stores the word of population I of node g where the next step reads it.
@@ -973,8 +950,8 @@ __device__ __forceinline__ RegSums reg_sums(const A &a, const Value &value, floa
     return t;
 }
 
-template <class S, bool SWAPPED, bool PERIODIC, int INTERIOR, class A>
-__device__ __forceinline__ void reg_relax_store(const A &a, const Node &g, const RegSums &t, const Shift &sh) {
+// The collision from the sums; put(K, f*_K, g*_K) takes the populations.
+template <class A, class Put> __device__ __forceinline__ void reg_relax(const A &a, const RegSums &t, const Put &put) {
     const Moments<float> &m = t.m;
     const float third = 1.f / 3.f;
     const float rho3 = mul_rn(m.rho, third);
@@ -990,14 +967,6 @@ __device__ __forceinline__ void reg_relax_store(const A &a, const Node &g, const
     const float uv = mul_rn(3.f, fma_rn(m.uz, m.uz, fma_rn(m.uy, m.uy, mul_rn(m.ux, m.ux))));
     const float kf = mul_rn(mul_rn(3.f, a.force_fac), mul_rn(a.gb, sub_rn(m.phi, a.t0)));
     const float k[3] = {mul_rn(kf, sub_rn(-1.f, m.uy)), mul_rn(kf, sub_rn(0.f, m.uy)), mul_rn(kf, sub_rn(1.f, m.uy))};
-    // population K's value out, normalised and relative to T_c where it goes
-    auto put = [&](auto kk, float fv, float gv) {
-        constexpr int K = decltype(kk)::value;
-        if (meets_plate<PERIODIC, INTERIOR, K>(g)) gv = abb<K>(gv, cy(K) < 0 ? a.t_hot : a.t_cold, m.rho);
-        const float sl = sub_rn(sh.s0, write_shift<SWAPPED, K, INTERIOR>(g, sh.t_dy));
-        store_word<S, SWAPPED, PERIODIC, INTERIOR, K>(
-            a, g, Pack16<S>::pack(mul_rn(fv, (float)winv(K)), fma_rn(gv, (float)winv(K), -sl)));
-    };
     {   // the rest population
         const float w = (float)wd(0);
         const float p = add_rn(0.f, mul_rn(0.5f, -uv));
@@ -1067,7 +1036,14 @@ __device__ __forceinline__ Moments<float> update_path16(const A &a, const Node &
             sink(t.m);
             const Node gs = again(a, g);
             a.phip[gs.n] = t.m.phi;
-            reg_relax_store<S, SWAPPED, PERIODIC, INTERIOR>(a, gs, t, sh);
+            // normalised and relative to T_c where it goes
+            reg_relax(a, t, [&](auto kk, float fv, float gv) {
+                constexpr int K = decltype(kk)::value;
+                if (meets_plate<PERIODIC, INTERIOR, K>(gs)) gv = abb<K>(gv, cy(K) < 0 ? a.t_hot : a.t_cold, t.m.rho);
+                const float sl = sub_rn(sh.s0, write_shift<SWAPPED, K, INTERIOR>(gs, sh.t_dy));
+                store_word<S, SWAPPED, PERIODIC, INTERIOR, K>(
+                    a, gs, Pack16<S>::pack(mul_rn(fv, (float)winv(K)), fma_rn(gv, (float)winv(K), -sl)));
+            });
         }
         return t.m;
     } else {
@@ -1109,47 +1085,72 @@ __device__ __forceinline__ Moments<float> step_moments16(const A &a, const Node 
     return update_node16<S, SWAPPED, PERIODIC, COLL, false>(a, g, NoMomentSink{});
 }
 
+// FP32 with the regularised collision, likewise: 54 values loaded, 18 sums
+// kept, two bodies.  B200, 256^3: 1112 us per step in the natural layout and
+// 1162 in the swapped one (0.99 of the copy rate), against 1636 and 1748 with
+// collide_reg, whose ~1100 FP32 operations per node bound it; bitwise its
+// results.
+template <bool SWAPPED, bool PERIODIC, int INTERIOR, class A, class Sink>
+__device__ __forceinline__ Moments<float> update_reg32(const A &a, const Node &g, const Sink &sink) {
+    const float phip = a.phip[g.n];
+    float fr[Q], gr[Q];
+    gather<float, SWAPPED, INTERIOR>(a, g, fr, gr);
+    const RegSums t = reg_sums(
+        a, [&](auto kk) { return make_float2(fr[decltype(kk)::value], gr[decltype(kk)::value]); }, phip);
+    sink(t.m);
+    const Node gs = again(a, g);
+    a.phip[gs.n] = t.m.phi;
+    reg_relax(a, t, [&](auto kk, float fv, float gv) {
+        constexpr int K = decltype(kk)::value;
+        if (meets_plate<PERIODIC, INTERIOR, K>(gs)) gv = abb<K>(gv, cy(K) < 0 ? a.t_hot : a.t_cold, t.m.rho);
+        store_pop<SWAPPED, INTERIOR, K>(a, gs, 0, fv);
+        store_pop<SWAPPED, INTERIOR, K>(a, gs, 1, gv);
+    });
+    return t.m;
+}
+
 template <class S, bool SWAPPED, bool PERIODIC, int COLL = LBM_COLLISION_BGK, class A, class Sink = NoMomentSink>
 __device__ __forceinline__ NodeOut<typename Codec<S>::R> update_node(const A &a, uint32_t n,
                                                                      const Sink &sink = Sink()) {
     if constexpr (sizeof(S) == 2) {
         const Node g = make_node<PERIODIC>(a, n);
         return {update_node16<S, SWAPPED, PERIODIC, COLL, true>(a, g, sink), g.iy};
+    } else if constexpr (sizeof(S) == 4 && COLL == LBM_COLLISION_REGULARIZED) {
+        const Node g = make_node<PERIODIC>(a, n);
+        return {yz_interior<PERIODIC>(g) ? update_reg32<SWAPPED, PERIODIC, kRowInside>(a, g, sink)
+                                         : update_reg32<SWAPPED, PERIODIC, kNoneInside>(a, g, sink),
+                g.iy};
     } else {
     using R = typename Codec<S>::R;
     const Node g = make_node<PERIODIC>(a, n);
     R fr[Q], gr[Q];
     // Rows away from the plates (and, in a closed box, from the z walls)
-    // need no y or z boundary tests, a closed box's warps with no x-wall
-    // node none at all, and in the swapped layout (the one whose accesses
-    // depend on them) the warps at one x wall test that side only; the
-    // path is uniform over a warp whenever LX is a multiple of 32.
-    constexpr bool kOneWall = SWAPPED && !PERIODIC;
-    const int path = kOneWall ? node_path_x<PERIODIC>(g) : node_path<PERIODIC, SWAPPED>(g);
-    if (!kOneWall && path == kRowInside)
+    // need no y or z boundary tests; the path is uniform over a warp whenever
+    // LX is a multiple of 32.  In FP32 a closed box's warps with no x-wall
+    // node take a body with no test at all in the swapped layout, the one
+    // whose accesses depend on them.  FP64 bodies are the longest, and a
+    // third one costs more in instruction fetches than its warps save (B200,
+    // 256^3 closed box, swapped step: 2334 us with two, 2370 with three, 2395
+    // with a body for each x wall too; FP32 1353, 1324 and 1368).
+    constexpr bool kThree = sizeof(S) == 4 && SWAPPED && !PERIODIC;
+    const int path = node_path<PERIODIC, kThree>(g);
+    if (path == kRowInside)
         gather<S, SWAPPED, kRowInside>(a, g, fr, gr);
-    else if (SWAPPED && !PERIODIC && path == kAllInside)
-        gather<S, SWAPPED, PERIODIC ? kRowInside : kAllInside>(a, g, fr, gr);
-    else if (kOneWall && path == kRowLoWall)
-        gather<S, SWAPPED, kOneWall ? kRowLoWall : kRowInside>(a, g, fr, gr);
-    else if (kOneWall && path == kRowHiWall)
-        gather<S, SWAPPED, kOneWall ? kRowHiWall : kRowInside>(a, g, fr, gr);
+    else if (kThree && path == kAllInside)
+        gather<S, SWAPPED, kThree ? kAllInside : kRowInside>(a, g, fr, gr);
     else
         gather<S, SWAPPED, kNoneInside>(a, g, fr, gr);
     const Moments<R> m = node_moments<S>(a, fr, gr, n);
     sink(m);
     collide<S, COLL>(fr, gr, m, a);
-    a.phip[n] = (typename Codec<S>::P)m.phi;
-    if (!kOneWall && path == kRowInside)
-        scatter<S, SWAPPED, PERIODIC, kRowInside>(a, g, fr, gr, m.rho);
-    else if (SWAPPED && !PERIODIC && path == kAllInside)
-        scatter<S, SWAPPED, PERIODIC, PERIODIC ? kRowInside : kAllInside>(a, g, fr, gr, m.rho);
-    else if (kOneWall && path == kRowLoWall)
-        scatter<S, SWAPPED, PERIODIC, kOneWall ? kRowLoWall : kRowInside>(a, g, fr, gr, m.rho);
-    else if (kOneWall && path == kRowHiWall)
-        scatter<S, SWAPPED, PERIODIC, kOneWall ? kRowHiWall : kRowInside>(a, g, fr, gr, m.rho);
+    const Node gs = again(a, g);
+    a.phip[gs.n] = (typename Codec<S>::P)m.phi;
+    if (path == kRowInside)
+        scatter<S, SWAPPED, PERIODIC, kRowInside>(a, gs, fr, gr, m.rho);
+    else if (kThree && path == kAllInside)
+        scatter<S, SWAPPED, PERIODIC, kThree ? kAllInside : kRowInside>(a, gs, fr, gr, m.rho);
     else
-        scatter<S, SWAPPED, PERIODIC, kNoneInside>(a, g, fr, gr, m.rho);
+        scatter<S, SWAPPED, PERIODIC, kNoneInside>(a, gs, fr, gr, m.rho);
     return {m, g.iy};
     }
 }
