@@ -291,7 +291,7 @@ int lbm_get_collision(const lbm_case *c, int32_t *model);
  * No counterpart in the reference, which runs one case per process.  A batch
  * holds cases (any grids, Ra, Pr) of one storage format, periodic sides, on
  * one device; it does not own them.  lbm_batch_step advances every member
- * by nsteps in one kernel launch per step (a CUDA graph of the launches is
+ * by nsteps in one kernel launch per step (per about 150 members) (a CUDA graph of the launches is
  * captured on first use of a step count and replayed); each member's step
  * count and layout advance as with lbm_step, and a member's result is the
  * same alone or in any mix; members may differ in collision model.  A case
@@ -319,7 +319,7 @@ int lbm_batch_step(lbm_batch *b, int32_t nsteps, void *stream);
  * lbm_get_observables per member (the reference reduces its one case on the
  * host, src/output.cu:148-280). */
 int lbm_batch_observables(lbm_batch *b, lbm_observables *out, void *stream);
-/* Launch shape: blocks of 128 or 256 threads, each tile 4 x block nodes of
+/* Launch shape: blocks of 128 or 256 threads, each tile as many nodes of
  * one member; blocks_per_sm > 0 runs that many persistent blocks per SM
  * walking the tile list, 0 one block per tile; use_graph replays captured
  * graphs for multi-step calls. */

@@ -3,12 +3,13 @@
 // A batch is a set of cases (any grids, Ra, Pr, collision models; one
 // storage format; periodic sides) on one device.  The members are grouped by
 // AA layout and collision model; one launch of batch_step_kernel per
-// non-empty group (normally one: members move through the layouts in step)
+// non-empty group (normally one: members move through the layouts in step;
+// more when a group has more members than one launch's parameters hold)
 // advances the group's members by one step.  Their nodes are cut into tiles
-// of kTileRounds x BLOCK nodes, numbered case after case; blocks walk the tile list with a
-// grid stride (persistent blocks, BLOCKS_PER_SM x 148 of them, or one block
-// per tile), find each tile's case by a binary search over the tiles' prefix
-// sums held in shared memory, and apply the same node update as the
+// of BLOCK nodes, numbered case after case; one block per tile, or
+// BLOCKS_PER_SM x 148 persistent blocks walking the tile list with a grid
+// stride, finds each tile's case by a binary search over the tiles' prefix
+// sums in the kernel parameters, and applies the same node update as the
 // single-case kernel (step.cuh update_node) with that case's parameters.  A
 // kernel instance holds the code of one layout and one model only, so it
 // needs no more registers than the single-case kernel.  A case's result
@@ -24,6 +25,7 @@
 #include <algorithm>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <new>
 #include <vector>
 
@@ -35,14 +37,8 @@ using namespace lbm_internal;
 
 namespace lbm {
 
-constexpr int kMaxBatch = 2048;    // members per batch (tile prefix sums in shared memory)
+constexpr int kMaxBatch = 2048;    // members per batch
 constexpr int kLanes = 8;          // streams of the one-kernel-per-member launch
-// A tile is kTileRounds rounds of BLOCK nodes of one member, so the member
-// lookup (binary search, descriptor) is paid once per kTileRounds nodes a
-// thread updates (96-case FP16S ensemble on B200: 19.3, 19.9, 20.5 and 20.6
-// GLUPS at 1, 2, 4 and 8 rounds; FP32 unchanged).
-constexpr int kTileRounds = 4;
-
 // Per-member descriptor, read by every block that works on the member.
 // It provides what update_node needs (the accessor interface of StepArgs).
 template <class S> struct BatchCase {
@@ -90,32 +86,46 @@ template <class S, int BLOCK, int COLL> struct BatchOccupancy {
     static constexpr int value = threads / BLOCK;
 };
 
-// Advances the members cases[0 .. ncases) of one group, all in layout
-// SWAPPED and collision model COLL, by one step.  tile_start[i] is the first
-// tile of member i (tile numbers are batch-wide; the group owns tiles
-// [tile_start[0], tile_start[ncases])).
-template <class S, int BLOCK, bool SWAPPED, int COLL>
+// What one launch of the batch kernel works on, passed by value: the kernel
+// parameters live in the constant bank, so a block finds its member (a binary
+// search over the tiles' prefix sums) and reads its descriptor without a
+// round trip to global memory or a barrier.
+template <class S, int MAX> struct BatchArgs {
+    uint32_t start[MAX + 1];   // first tile of member i (counted from the launch's first)
+    int32_t n;
+    BatchCase<S> cases[MAX];
+};
+
+// Members per launch: as many as the 32,764 bytes of kernel parameters hold,
+// or 32 (less to copy per launch).
+template <class S> constexpr int batch_max() { return (32764 - 64) / (int)(sizeof(BatchCase<S>) + 4); }
+constexpr int kBatchSmall = 32;
+
+// Advances the members of one launch, all in layout SWAPPED and collision
+// model COLL, by one step.  A tile is BLOCK nodes of one member, one per
+// thread.  With WALK persistent blocks walk the tiles; without, a block has
+// one tile and so never loads behind its own stores, which is what the
+// single-case kernel owes its speed to (step.cuh).  B200, 16 FP32 serving
+// cases: 2064 us per step, as their single-case kernels, against 2289 with
+// tiles of four rounds, descriptors in global memory and prefix sums copied
+// to shared memory by every block.
+template <class S, int BLOCK, bool SWAPPED, int COLL, int MAX, bool WALK>
 __global__ void __launch_bounds__(BLOCK, BatchOccupancy<S, BLOCK, COLL>::value)
-    batch_step_kernel(const BatchCase<S> *__restrict__ cases, int ncases, const uint32_t *__restrict__ tile_start) {
-    __shared__ uint32_t s_start[kMaxBatch + 1];
-    for (int i = threadIdx.x; i <= ncases; i += BLOCK) s_start[i] = tile_start[i];
-    __syncthreads();
-    const uint32_t end = s_start[ncases];
-    for (uint32_t t = s_start[0] + blockIdx.x; t < end; t += gridDim.x) {
-        int lo = 0, hi = ncases;   // the member c with s_start[c] <= t < s_start[c+1]
+    batch_step_kernel(const __grid_constant__ BatchArgs<S, MAX> b) {
+    const uint32_t end = b.start[b.n];
+    uint32_t t = blockIdx.x;
+    do {
+        int lo = 0, hi = b.n;   // the member c with start[c] <= t < start[c+1]
         while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
-            if (s_start[mid] <= t) lo = mid;
+            if (b.start[mid] <= t) lo = mid;
             else hi = mid;
         }
-        const BatchCase<S> &cs = cases[lo];
-        const uint32_t u0 = (t - s_start[lo]) * (BLOCK * kTileRounds) + threadIdx.x;
-#pragma unroll 1
-        for (int r = 0; r < kTileRounds; r++) {
-            const uint32_t u = u0 + r * BLOCK;
-            if (u < cs.nodes) update_node<S, SWAPPED, true, COLL>(cs, u);
-        }
-    }
+        const BatchCase<S> &cs = b.cases[lo];
+        const uint32_t u = (t - b.start[lo]) * BLOCK + threadIdx.x;
+        if (u < cs.nodes) update_node<S, SWAPPED, true, COLL>(cs, u);
+        t += gridDim.x;
+    } while (WALK && t < end);
 }
 
 }  // namespace lbm
@@ -127,26 +137,13 @@ struct lbm_batch {
     int32_t block = 128;           // tile size = threads per block
     int32_t blocks_per_sm = 0;     // 0: one block per tile
     bool use_graph = true;
-    // device copies of the descriptors and tile prefix sums
-    void *d_cases = nullptr;
-    uint32_t *d_start = nullptr;
-    int capacity = 0;
     // Member groups (descriptor order): bit 0 = the member's layout differs
     // from the batch's phase, bit 1 = regularised collision.  Every step
     // flips all layouts and the phase together, so groups stay fixed.
     int group_first[4] = {0, 0, 0, 0}, group_count[4] = {0, 0, 0, 0};
     int phase = 0;
-    bool dirty = true;             // descriptors need rebuilding / uploading
+    bool dirty = true;             // descriptors need rebuilding
     std::vector<unsigned char> h_cases;
-    std::vector<uint32_t> h_start;
-    // page-locked staging of the descriptor uploads, two in turn: an upload
-    // is a copy on the step stream that needs no wait, and a staging buffer
-    // is reused only after its event says its copy is done
-    unsigned char *stage[2] = {nullptr, nullptr};
-    size_t stage_cap[2] = {0, 0};
-    cudaEvent_t stage_ev[2] = {nullptr, nullptr};
-    bool stage_used[2] = {false, false};
-    int stage_next = 0;
     // lbm_batch_observables: one record per member (device)
     lbm_observables *d_obs = nullptr;
     int obs_cap = 0;
@@ -227,29 +224,11 @@ int group_of(const lbm_batch *b, const lbm_case *c) {
     return ((c->swapped ? 1 : 0) ^ b->phase) | (c->collision == LBM_COLLISION_REGULARIZED ? 2 : 0);
 }
 
-// Rebuilds and uploads the descriptors after a membership change.
-int refresh(lbm_batch *b, cudaStream_t st) {
+// Rebuilds the descriptors after a membership change.
+int refresh(lbm_batch *b) {
     if (!b->dirty) return LBM_OK;
     const int n = (int)b->members.size();
     const size_t db = case_desc_bytes(b->storage);
-    if (n > b->capacity) {
-        const int cap = std::max(n, std::max(16, 2 * b->capacity));
-        void *dc = nullptr;
-        uint32_t *ds = nullptr;
-        CUDA_TRY(cudaMalloc(&dc, (size_t)cap * db));
-        cudaError_t e = cudaMalloc(&ds, (size_t)(cap + 1) * sizeof(uint32_t));
-        if (e != cudaSuccess) {
-            cudaFree(dc);
-            return fail(LBM_ERR_NOMEM, "batch descriptor allocation failed");
-        }
-        CUDA_TRY(cudaStreamSynchronize(st));
-        cudaFree(b->d_cases);
-        cudaFree(b->d_start);
-        b->d_cases = dc;
-        b->d_start = ds;
-        b->capacity = cap;
-        drop_graphs(b);
-    }
     std::vector<const lbm_case *> order;
     order.reserve((size_t)n);
     for (int g = 0; g < 4; g++) {
@@ -259,45 +238,15 @@ int refresh(lbm_batch *b, cudaStream_t st) {
         b->group_count[g] = (int)order.size() - b->group_first[g];
     }
     b->h_cases.assign((size_t)n * db, 0);
-    b->h_start.assign((size_t)n + 1, 0);
-    uint32_t tiles = 0;
     int rc = with_batch_storage(b, [&](auto tag) {
         using S = std::remove_pointer_t<decltype(tag)>;
         for (int i = 0; i < n; i++) {
             const BatchCase<S> d = describe<S>(order[(size_t)i]);
             std::memcpy(b->h_cases.data() + (size_t)i * db, &d, db);
-            b->h_start[i] = tiles;
-            const int64_t tile = (int64_t)b->block * kTileRounds;
-            tiles += (uint32_t)((order[(size_t)i]->nodes + tile - 1) / tile);
         }
         return LBM_OK;
     });
     if (rc) return rc;
-    b->h_start[n] = tiles;
-    if (n > 0) {
-        // through page-locked staging: the copies run in stream order behind
-        // the steps already enqueued, and the host does not wait for them
-        const int i = b->stage_next;
-        const size_t cb = b->h_cases.size(), sb = b->h_start.size() * sizeof(uint32_t);
-        const size_t off = (cb + 255) / 256 * 256;
-        if (b->stage_used[i]) CUDA_TRY(cudaEventSynchronize(b->stage_ev[i]));
-        if (!b->stage_ev[i]) CUDA_TRY(cudaEventCreateWithFlags(&b->stage_ev[i], cudaEventDisableTiming));
-        if (b->stage_cap[i] < off + sb) {
-            if (b->stage[i]) cudaFreeHost(b->stage[i]);
-            b->stage[i] = nullptr;
-            b->stage_cap[i] = 0;
-            const size_t cap = std::max<size_t>(2 * (off + sb), 64 * 1024);
-            CUDA_TRY(cudaMallocHost((void **)&b->stage[i], cap));
-            b->stage_cap[i] = cap;
-        }
-        std::memcpy(b->stage[i], b->h_cases.data(), cb);
-        std::memcpy(b->stage[i] + off, b->h_start.data(), sb);
-        CUDA_TRY(cudaMemcpyAsync(b->d_cases, b->stage[i], cb, cudaMemcpyHostToDevice, st));
-        CUDA_TRY(cudaMemcpyAsync(b->d_start, b->stage[i] + off, sb, cudaMemcpyHostToDevice, st));
-        CUDA_TRY(cudaEventRecord(b->stage_ev[i], st));
-        b->stage_used[i] = true;
-        b->stage_next = 1 - i;
-    }
     b->dirty = false;
     return LBM_OK;
 }
@@ -307,10 +256,39 @@ unsigned grid_of(const lbm_batch *b, uint32_t tiles) {
     return (unsigned)std::min<uint64_t>(tiles, (uint64_t)b->sm_count * b->blocks_per_sm);
 }
 
+// One step of members [0, n) of one group (their descriptors at `d`), in
+// launches of at most MAX members.
+template <class S, int BLOCK, bool SW, int MAX>
+void launch_members(const lbm_batch *b, const unsigned char *d, int n, bool reg, cudaStream_t st) {
+    auto args = std::make_unique<BatchArgs<S, MAX>>();
+    for (int first = 0; first < n; first += MAX) {
+        args->n = std::min(MAX, n - first);
+        uint32_t tiles = 0;
+        for (int i = 0; i < args->n; i++) {
+            std::memcpy((void *)&args->cases[i], d + (size_t)(first + i) * sizeof(BatchCase<S>), sizeof(BatchCase<S>));
+            args->start[i] = tiles;
+            tiles += (args->cases[i].nodes + BLOCK - 1) / BLOCK;
+        }
+        args->start[args->n] = tiles;
+        auto launch = [&](auto walk) {
+            constexpr bool W = decltype(walk)::value;
+            const unsigned grid = grid_of(b, tiles);
+            if (reg) batch_step_kernel<S, BLOCK, SW, LBM_COLLISION_REGULARIZED, MAX, W><<<grid, BLOCK, 0, st>>>(*args);
+            else batch_step_kernel<S, BLOCK, SW, LBM_COLLISION_BGK, MAX, W><<<grid, BLOCK, 0, st>>>(*args);
+        };
+        if constexpr (MAX == batch_max<S>()) {
+            if (b->blocks_per_sm > 0) {
+                launch(std::true_type{});
+                continue;
+            }
+        }
+        launch(std::false_type{});
+    }
+}
 template <class S, int BLOCK, bool SW>
-void launch_group(const BatchCase<S> *cases, int n, const uint32_t *start, bool reg, unsigned grid, cudaStream_t st) {
-    if (reg) batch_step_kernel<S, BLOCK, SW, LBM_COLLISION_REGULARIZED><<<grid, BLOCK, 0, st>>>(cases, n, start);
-    else batch_step_kernel<S, BLOCK, SW, LBM_COLLISION_BGK><<<grid, BLOCK, 0, st>>>(cases, n, start);
+void launch_group(const lbm_batch *b, const unsigned char *d, int n, bool reg, cudaStream_t st) {
+    if (n <= kBatchSmall && b->blocks_per_sm <= 0) launch_members<S, BLOCK, SW, kBatchSmall>(b, d, n, reg, st);
+    else launch_members<S, BLOCK, SW, batch_max<S>()>(b, d, n, reg, st);
 }
 
 // Lane of each member for the per-case launch: members by decreasing node
@@ -371,24 +349,19 @@ int enqueue_steps(lbm_batch *b, int nsteps, cudaStream_t st) {
     if (b->launch == LBM_BATCH_PER_CASE) return enqueue_steps_per_case(b, nsteps, st);
     return with_batch_storage(b, [&](auto tag) {
         using S = std::remove_pointer_t<decltype(tag)>;
-        const BatchCase<S> *cases = (const BatchCase<S> *)b->d_cases;
         for (int s = 0; s < nsteps; s++)
             for (int g = 0; g < 4; g++) {
-                const int first = b->group_first[g], n = b->group_count[g];
+                const int n = b->group_count[g];
                 if (n == 0) continue;
-                const uint32_t tiles = b->h_start[first + n] - b->h_start[first];
-                const unsigned grid = grid_of(b, tiles);
-                if (grid == 0) continue;
+                const unsigned char *d = b->h_cases.data() + (size_t)b->group_first[g] * sizeof(BatchCase<S>);
                 const bool sw = ((g & 1) ^ b->phase ^ (s & 1)) != 0;
                 const bool reg = (g & 2) != 0;
-                const BatchCase<S> *c0 = cases + first;
-                const uint32_t *s0 = b->d_start + first;
                 if (b->block == 256) {
-                    if (sw) launch_group<S, 256, true>(c0, n, s0, reg, grid, st);
-                    else launch_group<S, 256, false>(c0, n, s0, reg, grid, st);
+                    if (sw) launch_group<S, 256, true>(b, d, n, reg, st);
+                    else launch_group<S, 256, false>(b, d, n, reg, st);
                 } else {
-                    if (sw) launch_group<S, 128, true>(c0, n, s0, reg, grid, st);
-                    else launch_group<S, 128, false>(c0, n, s0, reg, grid, st);
+                    if (sw) launch_group<S, 128, true>(b, d, n, reg, st);
+                    else launch_group<S, 128, false>(b, d, n, reg, st);
                 }
             }
         return LBM_OK;
@@ -443,21 +416,12 @@ int lbm_batch_destroy(lbm_batch *b) {
     for (lbm_case *m : b->members) m->batch = nullptr;
     DeviceGuard dg(b->device);
     drop_graphs(b);
-    cudaFree(b->d_cases);
-    cudaFree(b->d_start);
     cudaFree(b->d_obs);
     for (int l = 0; l < kLanes; l++) {
         if (b->lanes[l]) cudaStreamDestroy(b->lanes[l]);
         if (b->join_ev[l]) cudaEventDestroy(b->join_ev[l]);
     }
     if (b->fork_ev) cudaEventDestroy(b->fork_ev);
-    for (int i = 0; i < 2; i++) {
-        if (b->stage_ev[i]) {
-            cudaEventSynchronize(b->stage_ev[i]);
-            cudaEventDestroy(b->stage_ev[i]);
-        }
-        if (b->stage[i]) cudaFreeHost(b->stage[i]);
-    }
     if (b->capture_stream) cudaStreamDestroy(b->capture_stream);
     delete b;
     return LBM_OK;
@@ -508,7 +472,6 @@ int lbm_batch_set_config(lbm_batch *b, int32_t block, int32_t blocks_per_sm, int
     if (!b) return fail(LBM_ERR_ARG, "batch is NULL");
     if (block != 128 && block != 256) return fail(LBM_ERR_ARG, "block must be 128 or 256");
     if (blocks_per_sm < 0 || blocks_per_sm > 64) return fail(LBM_ERR_ARG, "blocks_per_sm must be 0..64");
-    if (block != b->block) b->dirty = true;
     b->block = block;
     b->blocks_per_sm = blocks_per_sm;
     b->use_graph = use_graph != 0;
@@ -544,7 +507,7 @@ int lbm_batch_step(lbm_batch *b, int32_t nsteps, void *stream) {
     if (nsteps == 0 || b->members.empty()) return LBM_OK;
     DeviceGuard dg(b->device);
     cudaStream_t st = (cudaStream_t)stream;
-    int rc = refresh(b, st);
+    int rc = refresh(b);
     if (rc) return rc;
     if (b->use_graph && nsteps > 1) {
         const int key = 2 * nsteps + b->phase;
