@@ -123,7 +123,10 @@ int lbm_derive(const lbm_params *p, lbm_derived *out);
  * temperature, reduction scratch), for admission against a memory budget.
  * The first lbm_step_observed call adds the rows of its in-kernel reduction
  * (13 doubles per 32 nodes, under 4 bytes per node) and one lbm_observables
- * per step of the longest call made. */
+ * per step of the longest call made; the first lbm_get_profile call adds at
+ * most 40 bytes per plane and 100 KB.  A case also holds a record of page-locked
+ * host memory, which lbm_get_observables' kernel writes; the library keeps
+ * them in pages of 4 KB, one of which it never frees. */
 int lbm_case_bytes(const lbm_params *p, uint64_t *bytes);
 
 /* Allocates a case on p->device (replaces the cudaMalloc calls of

@@ -563,7 +563,7 @@ int lbm_batch_observables(lbm_batch *b, lbm_observables *out, void *stream) {
     for (int i = 0; i < n; i++) {
         const lbm_case *c = b->members[(size_t)i];
         if (!c->initialised) return fail(LBM_ERR_STATE, "a member has no state");
-        const int rc = enqueue_observables(c, b->d_obs + i, st);
+        const int rc = enqueue_observables(c, b->d_obs + i, nullptr, st);
         if (rc) return rc;
     }
     CUDA_TRY(cudaGetLastError());

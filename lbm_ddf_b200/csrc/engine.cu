@@ -6,8 +6,8 @@
 //           ps = nodes rounded up to 128 elements so that every population
 //           row starts 256-byte aligned;
 //   phip  : previous-step temperature per node (FP64 for F64 storage, else FP32);
-//   scratch: per-block partial sums of the observables reduction and the
-//           reduced result.
+//   partial: per-block partial sums of the observables reduction, behind them
+//           the error flag and the reduction's count of finished blocks.
 // The layout flag `swapped` records which AA layout the populations are in.
 #include <cuda_runtime.h>
 
@@ -64,6 +64,59 @@ constexpr int kObsThreads = 256;
 // ---------------------------------------------------------------------------
 namespace lbm {
 
+struct ObsConsts {
+    double nodes, plane, ly, diff, dT, visc;
+    int64_t step;
+};
+
+// Sums the block partials in a fixed order (deterministic: warp w sums
+// quantity w, lane l the blocks l, l + 32, ..., then a butterfly over the
+// lanes) and forms the observables: Nu_bulk of src/output.cu:228-233;
+// Nu_top/bottom of :236-256 written with plane sums,
+// <(3T0 - 4T1 + T2)/2> = (3<T0> - 4<T1> + <T2>)/2.  For a block of any
+// number of warps (the quantities go round them); `partial` is read through
+// L2 (it may have been written by other blocks of the same launch).
+__device__ __forceinline__ void finalize_observables(const double *__restrict__ partial, int nblocks,
+                                                     const ObsConsts &c, lbm_observables *__restrict__ out) {
+    __shared__ double tot[kObs];
+    const int lane = threadIdx.x & 31;
+    for (int w = threadIdx.x >> 5; w < kObs; w += blockDim.x >> 5) {
+        double s = 0.0;
+        for (int b = lane; b < nblocks; b += 32) s += __ldcg(partial + (size_t)b * kObs + w);
+        s = warp_sum(s);
+        if (lane == 0) tot[w] = s;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const double uyT = tot[0] / c.nodes;
+        out->step = c.step;
+        out->nu_bulk = 1.0 + uyT * c.ly / (c.diff * c.dT);
+        const double b0 = tot[6] / c.plane, b1 = tot[7] / c.plane, b2 = tot[8] / c.plane;
+        const double t0 = tot[9] / c.plane, t1 = tot[10] / c.plane, t2 = tot[11] / c.plane;
+        const double dTdy_bot = (-3.0 * b0 + 4.0 * b1 - b2) / 2.0;
+        const double dTdy_top = (3.0 * t0 - 4.0 * t1 + t2) / 2.0;
+        out->nu_top = -dTdy_top * c.ly / c.dT;
+        out->nu_bottom = -dTdy_bot * c.ly / c.dT;
+        const double usq = tot[1] / c.nodes;
+        out->ke = 0.5 * usq;
+        out->re = sqrt(usq) * c.ly / c.visc;
+        out->ux_mean = tot[2] / c.nodes;
+        out->uy_mean = tot[3] / c.nodes;
+        out->uz_mean = tot[4] / c.nodes;
+        out->phi_mean = tot[5] / c.nodes;
+        out->diverged = tot[12] > 0.0 ? 1 : 0;
+        out->reserved = 0;
+    }
+}
+
+// Blocks per SM the reductions' registers are sized for.  Left to itself the
+// compiler takes 32 to 48 registers in the natural layout, loading each value
+// where it is added, with few in flight; at 2 blocks it has 128 and loads
+// ahead (B200, lbm_get_observables at 256^3: FP32 676 us natural and 638
+// swapped without a bound, 569 and 588 with; FP64 1320 and 1338, 1023 and
+// 1072).
+template <class S> constexpr int kObsMinBlocks = 2;
+
 // Per-block partial sums, in FP64, of
 //   0 uy*phi  1 |u|^2  2 ux  3 uy  4 uz  5 phi
 //   6..8  phi on the planes iy = 0, 1, 2
@@ -72,9 +125,18 @@ namespace lbm {
 //
 // 16-bit storage: the moments as the step of collision model `coll` forms
 // them, so these observables match those it reduces when it steps.
+//
+// With `done` (a count of finished blocks, 0 between launches) the block that
+// finishes last forms the observables too, so that reading a small case
+// costs one launch; `out` and `err_out`, the copy of the case's error flag,
+// may then be host memory the device can write, which saves the copies (B200,
+// 32^3 FP32: 45 us per lbm_get_observables with a second launch and two
+// copies, 23 with neither).  Without, obs_finalize follows.
 template <class S, bool SWAPPED, bool PERIODIC>
-__global__ void __launch_bounds__(kObsThreads) obs_kernel(const StepArgs<S> a, double *__restrict__ partial,
-                                                          int coll) {
+__global__ void __launch_bounds__(kObsThreads, kObsMinBlocks<S>) obs_kernel(const StepArgs<S> a, double *__restrict__ partial,
+                                                          int coll, unsigned *__restrict__ done, ObsConsts consts,
+                                                          lbm_observables *__restrict__ out, const int *err,
+                                                          int *err_out) {
     using R = typename Codec<S>::R;
     double acc[kObs];
 #pragma unroll
@@ -113,48 +175,17 @@ __global__ void __launch_bounds__(kObsThreads) obs_kernel(const StepArgs<S> a, d
         for (int w = 0; w < kObsThreads / 32; w++) s += red[threadIdx.x][w];
         partial[(size_t)blockIdx.x * kObs + threadIdx.x] = s;
     }
-}
-
-struct ObsConsts {
-    double nodes, plane, ly, diff, dT, visc;
-    int64_t step;
-};
-
-// Sums the block partials in a fixed order (deterministic: warp w sums
-// quantity w, lane l the blocks l, l + 32, ..., then a butterfly over the
-// lanes) and forms the observables: Nu_bulk of src/output.cu:228-233;
-// Nu_top/bottom of :236-256 written with plane sums,
-// <(3T0 - 4T1 + T2)/2> = (3<T0> - 4<T1> + <T2>)/2.  Launch: kObs warps.
-// The body of obs_finalize, for a block of kObs warps; `partial` is read
-// through L2 (it may have been written by other blocks of the same launch).
-__device__ __forceinline__ void finalize_observables(const double *__restrict__ partial, int nblocks,
-                                                     const ObsConsts &c, lbm_observables *__restrict__ out) {
-    __shared__ double tot[kObs];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double s = 0.0;
-    for (int b = lane; b < nblocks; b += 32) s += __ldcg(partial + (size_t)b * kObs + w);
-    s = warp_sum(s);
-    if (lane == 0) tot[w] = s;
+    if (!done) return;
+    __shared__ bool last;
+    __threadfence();
     __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    finalize_observables(partial, gridDim.x, consts, out);
     if (threadIdx.x == 0) {
-        const double uyT = tot[0] / c.nodes;
-        out->step = c.step;
-        out->nu_bulk = 1.0 + uyT * c.ly / (c.diff * c.dT);
-        const double b0 = tot[6] / c.plane, b1 = tot[7] / c.plane, b2 = tot[8] / c.plane;
-        const double t0 = tot[9] / c.plane, t1 = tot[10] / c.plane, t2 = tot[11] / c.plane;
-        const double dTdy_bot = (-3.0 * b0 + 4.0 * b1 - b2) / 2.0;
-        const double dTdy_top = (3.0 * t0 - 4.0 * t1 + t2) / 2.0;
-        out->nu_top = -dTdy_top * c.ly / c.dT;
-        out->nu_bottom = -dTdy_bot * c.ly / c.dT;
-        const double usq = tot[1] / c.nodes;
-        out->ke = 0.5 * usq;
-        out->re = sqrt(usq) * c.ly / c.visc;
-        out->ux_mean = tot[2] / c.nodes;
-        out->uy_mean = tot[3] / c.nodes;
-        out->uz_mean = tot[4] / c.nodes;
-        out->phi_mean = tot[5] / c.nodes;
-        out->diverged = tot[12] > 0.0 ? 1 : 0;
-        out->reserved = 0;
+        *done = 0u;
+        if (err_out) *err_out = *err;
     }
 }
 
@@ -198,19 +229,31 @@ __global__ void __launch_bounds__(32 * kObs) obs_rows_reduce(const double *__res
     if (t == 0) *done = 0u;
 }
 
-// Vertical profile, src/output.cu:336-368: one block per xz plane iy.
+// Vertical profile, src/output.cu:336-368: block b sums a chunk of the xz
+// plane iy = b / chunks into partial[b], profile_finalize adds a plane's
+// chunks in order.  Enough chunks that the grid fills the device: one block
+// per plane left most of it idle (B200: 3.4 ms at 256^3 FP32 and 4.25 ms at
+// 512x256x512 FP16S, 0.61 and 1.25 now; a read of the state takes 0.56 and
+// 1.15).
+constexpr int kProf = 5;
 template <class S, bool SWAPPED, bool PERIODIC>
-__global__ void __launch_bounds__(kObsThreads) profile_kernel(const StepArgs<S> a, double *__restrict__ out) {
+__global__ void __launch_bounds__(kObsThreads, kObsMinBlocks<S> + (sizeof(S) == 2)) profile_kernel(const StepArgs<S> a, uint32_t chunks,
+                                                              double *__restrict__ partial) {
     using R = typename Codec<S>::R;
-    const int iy = blockIdx.x;
-    double acc[5] = {0, 0, 0, 0, 0};
+    const uint32_t iy = blockIdx.x / chunks, chunk = blockIdx.x - iy * chunks;
+    double acc[kProf] = {0, 0, 0, 0, 0};
     const uint32_t cnt = (uint32_t)a.lx * (uint32_t)a.lz;
-    for (uint32_t t = threadIdx.x; t < cnt; t += blockDim.x) {
-        const uint32_t iz = t / (uint32_t)a.lx, ix = t - iz * (uint32_t)a.lx;
-        const uint32_t n = (iz * (uint32_t)a.ly + (uint32_t)iy) * (uint32_t)a.lx + ix;
+    const uint32_t per = (cnt + chunks - 1) / chunks;
+    const uint32_t end = min(cnt, (chunk + 1) * per);
+    for (uint32_t t = chunk * per + threadIdx.x; t < end; t += kObsThreads) {
+        const uint32_t iz = a.div_lx.div(t), ix = t - iz * (uint32_t)a.lx;
+        const uint32_t n = (iz * (uint32_t)a.ly + iy) * (uint32_t)a.lx + ix;
         const Node g = make_node<PERIODIC>(a, n);
         R fr[Q], gr[Q];
-        gather<S, SWAPPED>(a, g, fr, gr);
+        if (SWAPPED && yz_interior<PERIODIC>(g))
+            gather<S, SWAPPED, kRowInside>(a, g, fr, gr);
+        else
+            gather<S, SWAPPED, kNoneInside>(a, g, fr, gr);
         const Moments<R> m = node_moments<S>(a, fr, gr, n);
         acc[0] += (double)m.ux;
         acc[1] += (double)m.uy;
@@ -218,28 +261,36 @@ __global__ void __launch_bounds__(kObsThreads) profile_kernel(const StepArgs<S> 
         acc[3] += (double)m.phi;
         acc[4] += (double)m.phi * (double)m.phi;
     }
-    __shared__ double red[5][kObsThreads / 32];
+    __shared__ double red[kProf][kObsThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int k = 0; k < 5; k++) {
+    for (int k = 0; k < kProf; k++) {
         double v = warp_sum(acc[k]);
         if (lane == 0) red[k][warp] = v;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double s[5];
-        for (int k = 0; k < 5; k++) {
-            s[k] = 0.0;
-            for (int w = 0; w < (int)(blockDim.x / 32); w++) s[k] += red[k][w];
-        }
-        const double c = (double)cnt;
-        const double ap = s[3] / c;
-        out[5 * iy + 0] = s[0] / c;
-        out[5 * iy + 1] = s[1] / c;
-        out[5 * iy + 2] = s[2] / c;
-        out[5 * iy + 3] = ap;
-        out[5 * iy + 4] = sqrt(s[4] / c - ap * ap);
+    if (threadIdx.x < kProf) {
+        double s = 0.0;
+        for (int w = 0; w < kObsThreads / 32; w++) s += red[threadIdx.x][w];
+        partial[(size_t)blockIdx.x * kProf + threadIdx.x] = s;
     }
+}
+
+// One thread per plane.
+__global__ void profile_finalize(const double *__restrict__ partial, uint32_t chunks, int ly, double cnt,
+                                 double *__restrict__ out) {
+    const int iy = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (iy >= ly) return;
+    double s[kProf] = {0, 0, 0, 0, 0};
+    for (uint32_t c = 0; c < chunks; c++)
+        for (int k = 0; k < kProf; k++) s[k] += partial[((size_t)iy * chunks + c) * kProf + k];
+    double *o = out + (size_t)iy * kProf;
+    const double ap = s[3] / cnt;
+    o[0] = s[0] / cnt;
+    o[1] = s[1] / cnt;
+    o[2] = s[2] / cnt;
+    o[3] = ap;
+    o[4] = sqrt(s[4] / cnt - ap * ap);
 }
 
 // One population (which 0 = f, 1 = g; index k), decoded, natural order.
@@ -605,14 +656,76 @@ template <class S, bool SW, bool PER> int obs_resident() {
     return resident;
 }
 template <class S>
-int launch_obs(const lbm_case *c, const StepArgs<S> &a, double *partial, int cap, int sms, int coll,
-               cudaStream_t st) {
+int launch_obs(const lbm_case *c, const StepArgs<S> &a, double *partial, int cap, int sms, int coll, unsigned *done,
+               const ObsConsts &k, lbm_observables *out, const int *err, int *err_out, cudaStream_t st) {
     const bool per = c->p.sides == LBM_SIDES_PERIODIC;
     const int resident = c->swapped ? (per ? obs_resident<S, true, true>() : obs_resident<S, true, false>())
                                     : (per ? obs_resident<S, false, true>() : obs_resident<S, false, false>());
     const int blocks = std::max(1, std::min(cap, sms * resident));
-    LBM_DISPATCH_LAYOUT(c, obs_kernel, blocks, kObsThreads, st, a, partial, coll);
+    LBM_DISPATCH_LAYOUT(c, obs_kernel, blocks, kObsThreads, st, a, partial, coll, done, k, out, err, err_out);
     return blocks;
+}
+
+// Page-locked host records of the live cases, in pages of 32 (allocating and
+// freeing one costs ~0.6 ms, more than creating a small case).  A page whose
+// records are all back is freed unless it is the only one, so beyond one page
+// the memory follows the number of live cases.
+struct RecordPage {
+    struct alignas(128) Slot {
+        HostRecord rec;
+    };
+    Slot *slots = nullptr;
+    uint32_t used = 0;   // bit i: slot i is taken
+};
+constexpr int kPageSlots = 32;
+std::mutex g_records_mu;
+std::vector<RecordPage> g_records;
+
+cudaError_t take_record(HostRecord **out) {
+    std::lock_guard<std::mutex> lk(g_records_mu);
+    for (RecordPage &p : g_records)
+        for (int i = 0; i < kPageSlots; i++)
+            if (!(p.used >> i & 1u)) {
+                p.used |= 1u << i;
+                *out = &p.slots[i].rec;
+                return cudaSuccess;
+            }
+    RecordPage p;
+    const cudaError_t e =
+        cudaHostAlloc((void **)&p.slots, kPageSlots * sizeof(RecordPage::Slot), cudaHostAllocPortable);
+    if (e != cudaSuccess) return e;
+    p.used = 1u;
+    *out = &p.slots[0].rec;
+    g_records.push_back(p);
+    return cudaSuccess;
+}
+
+void give_record(HostRecord *r) {
+    if (!r) return;
+    std::lock_guard<std::mutex> lk(g_records_mu);
+    for (size_t k = 0; k < g_records.size(); k++) {
+        RecordPage &p = g_records[k];
+        const auto *slot = reinterpret_cast<const RecordPage::Slot *>(r);
+        if (slot < p.slots || slot >= p.slots + kPageSlots) continue;
+        p.used &= ~(1u << (slot - p.slots));
+        if (p.used == 0 && g_records.size() > 1) {
+            cudaFreeHost(p.slots);
+            g_records.erase(g_records.begin() + (std::ptrdiff_t)k);
+        }
+        return;
+    }
+}
+
+ObsConsts obs_consts(const lbm_case *c, int64_t step) {
+    ObsConsts k;
+    k.nodes = (double)c->nodes;
+    k.plane = (double)c->p.lx * (double)c->p.lz;
+    k.ly = (double)c->p.ly;
+    k.diff = c->d.diff;
+    k.dT = c->p.t_hot - c->p.t_cold;
+    k.visc = c->d.visc;
+    k.step = step;
+    return k;
 }
 
 int check_case(const lbm_case *c, bool need_state) {
@@ -688,10 +801,15 @@ int lbm_create(const lbm_params *p, lbm_case **out) {
         if (e == cudaSuccess) e = cudaMalloc(&c->g, pop_bytes);
     }
     if (e == cudaSuccess) e = cudaMalloc(&c->phip, carry_bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&c->partial, (size_t)c->obs_blocks * kObs * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&c->d_obs, sizeof(lbm_observables));
-    if (e == cudaSuccess) e = cudaMalloc(&c->d_err, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(c->d_err, 0, sizeof(int));
+    // the reduction rows, then the error flag and the count of finished blocks
+    const size_t rows = (size_t)c->obs_blocks * kObs * sizeof(double);
+    if (e == cudaSuccess) e = cudaMalloc(&c->partial, rows + 2 * sizeof(int));
+    if (e == cudaSuccess) {
+        c->d_err = (int *)((char *)c->partial + rows);
+        c->obs_done = (unsigned *)(c->d_err + 1);
+        e = cudaMemset(c->d_err, 0, 2 * sizeof(int));
+    }
+    if (e == cudaSuccess) e = take_record(&c->host);
     if (e != cudaSuccess) {
         cudaGetLastError();
         lbm_destroy(c);
@@ -710,8 +828,8 @@ int lbm_destroy(lbm_case *c) {
     if (!interleaved(c)) cudaFree(c->g);
     cudaFree(c->phip);
     cudaFree(c->partial);
-    cudaFree(c->d_obs);
-    cudaFree(c->d_err);
+    give_record(c->host);
+    cudaFree(c->prof);
     cudaFree(c->obs_rows);
     cudaFree(c->obs_series);
     delete c;
@@ -917,21 +1035,14 @@ int lbm_step(lbm_case *c, int32_t nsteps, void *stream) {
 }  // extern "C"
 
 // Enqueues on `st` the observables reduction of case c's current state into
-// dst (device memory): two kernels, no synchronisation.
-int lbm_internal::enqueue_observables(const lbm_case *c, lbm_observables *dst, cudaStream_t st) {
+// dst (memory the device can write; err_out, if given, takes the case's error
+// flag): one kernel, no synchronisation.
+int lbm_internal::enqueue_observables(const lbm_case *c, lbm_observables *dst, int *err_out, cudaStream_t st) {
     return with_storage(c, [&](auto tag) {
         using S = std::remove_pointer_t<decltype(tag)>;
         const StepArgs<S> a = make_args<S>(c);
-        const int blocks = launch_obs<S>(c, a, c->partial, c->obs_blocks, c->sms, c->collision, st);
-        ObsConsts k;
-        k.nodes = (double)c->nodes;
-        k.plane = (double)c->p.lx * (double)c->p.lz;
-        k.ly = (double)c->p.ly;
-        k.diff = c->d.diff;
-        k.dT = c->p.t_hot - c->p.t_cold;
-        k.visc = c->d.visc;
-        k.step = c->step;
-        obs_finalize<<<1, 32 * kObs, 0, st>>>(c->partial, blocks, k, dst);
+        launch_obs<S>(c, a, c->partial, c->obs_blocks, c->sms, c->collision, c->obs_done, obs_consts(c, c->step), dst,
+                      c->d_err, err_out, st);
         return LBM_OK;
     });
 }
@@ -965,13 +1076,13 @@ int lbm_get_observables(lbm_case *c, lbm_observables *out, void *stream) {
     if (!out) return fail(LBM_ERR_ARG, "out is NULL");
     DeviceGuard dg(c->p.device);
     cudaStream_t st = (cudaStream_t)stream;
-    rc = enqueue_observables(c, c->d_obs, st);
+    // the kernel writes the record to page-locked memory of the case
+    rc = enqueue_observables(c, &c->host->obs, &c->host->err, st);
     if (rc) return rc;
     CUDA_TRY(cudaGetLastError());
-    CUDA_TRY(cudaMemcpyAsync(out, c->d_obs, sizeof(lbm_observables), cudaMemcpyDeviceToHost, st));
-    int err = 0;
-    CUDA_TRY(cudaMemcpyAsync(&err, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
+    *out = c->host->obs;
+    const int err = c->host->err;
     if (err) return fail(LBM_ERR_CUDA, "a step kernel gave up waiting for its shared-memory copies");
     if (out->diverged) return fail(LBM_ERR_DIVERGED, "NaN/Inf in the macroscopic fields");
     return LBM_OK;
@@ -1011,13 +1122,7 @@ static int step_observed(lbm_case *c, int32_t nsteps, lbm_observables *out, void
         using S = std::remove_pointer_t<decltype(tag)>;
         StepArgs<S> a = make_args<S>(c);
         a.obs_rows = c->obs_rows;
-        ObsConsts k;
-        k.nodes = (double)c->nodes;
-        k.plane = (double)c->p.lx * (double)c->p.lz;
-        k.ly = (double)c->p.ly;
-        k.diff = c->d.diff;
-        k.dT = c->p.t_hot - c->p.t_cold;
-        k.visc = c->d.visc;
+        ObsConsts k = obs_consts(c, c->step);
         for (int s = 0; s < nsteps; s++) {
             k.step = c->step + s;   // the state this step starts from
             launch_step_observed<S>(c, a, st);
@@ -1054,21 +1159,24 @@ int lbm_get_profile(lbm_case *c, double *out, void *stream) {
     if (!out) return fail(LBM_ERR_ARG, "out is NULL");
     DeviceGuard dg(c->p.device);
     cudaStream_t st = (cudaStream_t)stream;
-    double *dprof = nullptr;
-    CUDA_TRY(cudaMalloc(&dprof, (size_t)5 * c->p.ly * sizeof(double)));
+    const int64_t cnt = (int64_t)c->p.lx * c->p.lz, ly = c->p.ly;
+    // chunks per plane: about 16 blocks per SM over all planes, a chunk no
+    // smaller than a block
+    const int64_t chunks = std::max<int64_t>(
+        1, std::min<int64_t>((cnt + kObsThreads - 1) / kObsThreads, ((int64_t)c->sms * 16 + ly - 1) / ly));
+    if (!c->prof) CUDA_TRY(cudaMalloc(&c->prof, (size_t)(ly * chunks + ly) * kProf * sizeof(double)));
+    double *dprof = c->prof + (size_t)(ly * chunks) * kProf;
     rc = with_storage(c, [&](auto tag) {
         using S = std::remove_pointer_t<decltype(tag)>;
         const StepArgs<S> a = make_args<S>(c);
-        LBM_DISPATCH_LAYOUT(c, profile_kernel, c->p.ly, kObsThreads, st, a, dprof);
+        LBM_DISPATCH_LAYOUT(c, profile_kernel, (unsigned)(ly * chunks), kObsThreads, st, a, (uint32_t)chunks, c->prof);
         return LBM_OK;
     });
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(out, dprof, (size_t)5 * c->p.ly * sizeof(double), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFree(dprof);
     if (rc) return rc;
-    if (e != cudaSuccess) return fail(LBM_ERR_CUDA, cudaGetErrorString(e));
+    profile_finalize<<<grid_for(ly, 128), 128, 0, st>>>(c->prof, (uint32_t)chunks, (int)ly, (double)cnt, dprof);
+    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(cudaMemcpyAsync(out, dprof, (size_t)kProf * ly * sizeof(double), cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaStreamSynchronize(st));
     return LBM_OK;
 }
 
@@ -1241,15 +1349,11 @@ int lbm_observables_noalloc(const lbm_params *p, const void *f, const void *g, c
         const StepArgs<S> a = make_args<S>(&view);
         const lbm_case *c = &view;
         // 16-bit storage: the moments as the BGK step forms them
-        const int blocks = launch_obs<S>(c, a, scratch, cap, sms, LBM_COLLISION_BGK, st);
-        ObsConsts k;
-        k.nodes = (double)nodes;
-        k.plane = (double)p->lx * (double)p->lz;
-        k.ly = (double)p->ly;
-        k.diff = view.d.diff;
-        k.dT = p->t_hot - p->t_cold;
-        k.visc = view.d.visc;
-        k.step = step;
+        // two kernels: a count of finished blocks would outlive a call that
+        // overlaps another, as the rows need not
+        const ObsConsts k = obs_consts(c, step);
+        const int blocks = launch_obs<S>(c, a, scratch, cap, sms, LBM_COLLISION_BGK, nullptr, k, nullptr, nullptr,
+                                         nullptr, st);
         obs_finalize<<<1, 32 * kObs, 0, st>>>(scratch, blocks, k, out_dev);
         return LBM_OK;
     });

@@ -9,6 +9,12 @@
 
 #include "../../include/lbm_ddf.h"
 
+// observables and error flag of a case, written by the device to host memory
+struct HostRecord {
+    lbm_observables obs;
+    int32_t err;
+};
+
 struct lbm_case {
     lbm_params p;
     lbm_derived d;
@@ -23,10 +29,12 @@ struct lbm_case {
     int32_t kernel = LBM_KERNEL_AUTO;    // step kernel choice
     int32_t collision = LBM_COLLISION_BGK;
     lbm_batch *batch = nullptr;          // the batch the case is a member of
-    int *d_err = nullptr;                // set by a step kernel whose bulk-copy wait timed out
+    int *d_err = nullptr;                // set by a step kernel whose bulk-copy wait timed out (behind partial)
     uint32_t debug_extra_tx = 0;         // lbm_debug_row_wait_extra_bytes (0: off)
     double *partial = nullptr;           // obs partial sums
-    lbm_observables *d_obs = nullptr;    // reduced observables (device)
+    unsigned *obs_done = nullptr;        // blocks of the reduction that are done (behind partial)
+    HostRecord *host = nullptr;          // what lbm_get_observables' kernel writes (page-locked)
+    double *prof = nullptr;              // lbm_get_profile: chunk sums and the profile, from its first call
     int obs_blocks = 0;                  // partial rows (most reduction blocks)
     int sms = 148;                       // SM count of the case's device
     double *obs_rows = nullptr;          // lbm_step_observed: per-warp rows + chunk partials
@@ -49,9 +57,10 @@ void derive(const lbm_params *p, lbm_derived *d);
 int check_params(const lbm_params *p);
 // drops a case that is being destroyed from its batch (batch.cu)
 void batch_forget(lbm_batch *b, lbm_case *c);
-// enqueues the observables reduction of c's current state into dst (device
-// memory) on st, without synchronising (engine.cu)
-int enqueue_observables(const lbm_case *c, lbm_observables *dst, cudaStream_t st);
+// enqueues the observables reduction of c's current state into dst (memory
+// the device can write), and the error flag into err_out if given, on st,
+// without synchronising (engine.cu)
+int enqueue_observables(const lbm_case *c, lbm_observables *dst, int *err_out, cudaStream_t st);
 // enqueues one node-kernel step of c from layout `swapped` on st; the host
 // state (step count, layout flag) is the caller's to advance (engine.cu)
 int enqueue_case_step(const lbm_case *c, bool swapped, cudaStream_t st);
