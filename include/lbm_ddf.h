@@ -122,7 +122,7 @@ int lbm_derive(const lbm_params *p, lbm_derived *out);
 /* Device bytes a case with these parameters holds (populations, carried
  * temperature, reduction scratch), for admission against a memory budget.
  * The first lbm_step_observed call adds the rows of its in-kernel reduction
- * (13 doubles per 32 nodes, under 4 bytes per node) and one lbm_observables
+ * (14 doubles per 32 nodes, under 4 bytes per node) and one lbm_observables
  * per step of the longest call made; the first lbm_get_profile call adds at
  * most 40 bytes per plane and 100 KB.  A case also holds a record of page-locked
  * host memory, which lbm_get_observables' kernel writes; the library keeps

@@ -194,32 +194,54 @@ __global__ void __launch_bounds__(32 * kObs) obs_finalize(const double *__restri
     finalize_observables(partial, nblocks, c, out);
 }
 
-// The per-warp rows a fused step kernel wrote, summed in blocks of
-// kRowChunk rows into one partial row each, then (by the block that finishes
-// last) the partial rows into the observables, as obs_finalize forms them.
-// Thread t of a block reads the chunk's words t, t + 32 kObs, ...: coalesced,
-// and all of term t % kObs, rows t / kObs + 32 i; the 32 threads of a term
-// are then added by a butterfly in row order.  A fixed order, so the result
-// is deterministic.  `done` counts the blocks that have written their
-// partial row; the last one resets it to 0 for the next launch.  Launch: kObs
-// warps per block.
-constexpr int kRowChunk = 1024;
-__global__ void __launch_bounds__(32 * kObs) obs_rows_reduce(const double *__restrict__ rows, int nrows,
-                                                             double *__restrict__ partial,
-                                                             unsigned *__restrict__ done, ObsConsts c,
-                                                             lbm_observables *__restrict__ out) {
-    __shared__ double red[32 * kObs];
+// The rows an observed step's warps wrote (step.cuh warp_obs_row), summed in
+// chunks into one partial row of kObs terms each, then (by the block that
+// finishes last) the partial rows into the observables, as obs_finalize forms
+// them.  Thread t takes word t % kObsRow of the chunk's rows t / kObsRow + 32 i
+// (coalesced); the phi thread also finds its rows' plane terms.  The 32 threads
+// of a term are then added in row order: a fixed order, so the result is
+// deterministic.  `done` counts the blocks that have written their partial
+// row; the last one resets it to 0 for the next launch.
+constexpr int kRowThreads = 32 * kObsRow;
+struct RowGeometry {
+    FastDiv div_lx, div_ly;
+    int32_t ly;
+    uint32_t nodes;
+};
+__global__ void __launch_bounds__(kRowThreads) obs_rows_reduce(const double *__restrict__ rows,
+                                                               const double *__restrict__ planes, int nrows, int chunk,
+                                                               RowGeometry geo, double *__restrict__ partial,
+                                                               unsigned *__restrict__ done, ObsConsts c,
+                                                               lbm_observables *__restrict__ out) {
+    __shared__ double red[kObs][32];
     __shared__ bool last;
-    const int t = threadIdx.x, w = t >> 5, lane = t & 31;
-    const int r0 = blockIdx.x * kRowChunk;
-    const int words = (min(nrows, r0 + kRowChunk) - r0) * kObs;
-    const double *chunk = rows + (size_t)r0 * kObs;
-    double s = 0.0;
-    for (int e = t; e < words; e += 32 * kObs) s += chunk[e];
-    red[t] = s;
+    const int t = threadIdx.x, word = t % kObsRow, r0 = blockIdx.x * chunk, r1 = min(nrows, r0 + chunk);
+    double s = 0.0, p[kObsPlanes] = {};
+    for (int r = r0 + t / kObsRow; r < r1; r += 32) {
+        const double v = rows[(size_t)r * kObsRow + word];
+        s += v;
+        if (word == 5) {
+            const uint32_t first = 32u * (uint32_t)r, end = min(geo.nodes - 1u, first + 31u);
+            const uint32_t q0 = geo.div_lx.div(first), span = geo.div_lx.div(end) - q0;
+            const int iy0 = (int)(q0 - geo.div_ly.div(q0) * (uint32_t)geo.ly);
+            if (iy0 <= 2 || iy0 + (int)span >= geo.ly - 3) {
+#pragma unroll
+                for (int k = 0; k < kObsPlanes; k++)
+                    p[k] += span ? planes[(size_t)r * kObsPlanes + k]
+                                 : iy0 == (k < 3 ? k : geo.ly - 1 - (k - 3)) ? v : 0.0;
+            }
+        }
+    }
+    if (word < 6) red[word][t / kObsRow] = s;
+    if (word == 6) red[12][t / kObsRow] = s;
+    if (word == 5)
+        for (int k = 0; k < kObsPlanes; k++) red[6 + k][t / kObsRow] = p[k];
     __syncthreads();
-    const double v = warp_sum(red[lane * kObs + w]);   // term w, rows lane + 32 i
-    if (lane == 0) partial[(size_t)blockIdx.x * kObs + w] = v;
+    const int w = t >> 5, lane = t & 31;
+    for (int k = w; k < kObs; k += kRowThreads / 32) {
+        const double v = warp_sum(red[k][lane]);
+        if (lane == 0) partial[(size_t)blockIdx.x * kObs + k] = v;
+    }
     __threadfence();
     __syncthreads();
     if (t == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
@@ -498,7 +520,7 @@ template <class S> StepArgs<S> make_args(const lbm_case *c) {
         a.pairs[b] = a.pairs_st[b] = (S *)c->f + (size_t)(9 * b) * (size_t)c->ps * elem_stride<S>();
     a.pair_row = a.pair_row_st = (uint32_t)c->ps;
     a.zero = 0;
-    a.obs_rows = nullptr;
+    a.obs_rows = a.obs_planes = nullptr;
     a.phip = (typename Codec<S>::P *)c->phip;
     a.lx = c->p.lx;
     a.ly = c->p.ly;
@@ -1100,11 +1122,14 @@ static int step_observed(lbm_case *c, int32_t nsteps, lbm_observables *out, void
     DeviceGuard dg(c->p.device);
     cudaStream_t st = (cudaStream_t)stream;
     const int rows = obs_rows_of(c);   // one per warp of the node kernel
-    const int parts = (rows + kRowChunk - 1) / kRowChunk;
-    if (!c->obs_rows) {   // per-warp rows, the chunk partials, the count of chunks done
-        const size_t bytes = (size_t)(rows + parts) * kObs * sizeof(double);
-        CUDA_TRY(cudaMalloc(&c->obs_rows, bytes + sizeof(double)));
-        CUDA_TRY(cudaMemsetAsync((char *)c->obs_rows + bytes, 0, sizeof(double), st));
+    // rows per block of their reduction: two blocks per SM or more, but at
+    // most 1024 rows, so that few partial rows are left
+    const int chunk = std::min(1024, std::max(64, (rows + 2 * c->sms - 1) / (2 * c->sms)));
+    const int parts = (rows + chunk - 1) / chunk;
+    const size_t words = (size_t)rows * (kObsRow + kObsPlanes) + (size_t)parts * kObs;
+    if (!c->obs_rows) {   // rows, plane sums, the chunk partials, the count of chunks done
+        CUDA_TRY(cudaMalloc(&c->obs_rows, (words + 1) * sizeof(double)));
+        CUDA_TRY(cudaMemsetAsync(c->obs_rows + words, 0, sizeof(double), st));
     }
     if (nsteps > c->obs_series_cap) {
         if (c->obs_series) {
@@ -1116,17 +1141,21 @@ static int step_observed(lbm_case *c, int32_t nsteps, lbm_observables *out, void
         CUDA_TRY(cudaMalloc(&c->obs_series, (size_t)nsteps * sizeof(lbm_observables)));
         c->obs_series_cap = nsteps;
     }
-    double *partial = c->obs_rows + (size_t)rows * kObs;
-    unsigned *done = (unsigned *)(partial + (size_t)parts * kObs);
+    double *planes = c->obs_rows + (size_t)rows * kObsRow;
+    double *partial = planes + (size_t)rows * kObsPlanes;
+    unsigned *done = (unsigned *)(c->obs_rows + words);
     rc = with_storage(c, [&](auto tag) {
         using S = std::remove_pointer_t<decltype(tag)>;
         StepArgs<S> a = make_args<S>(c);
         a.obs_rows = c->obs_rows;
+        a.obs_planes = planes;
+        const RowGeometry geo = {a.div_lx, a.div_ly, a.ly, a.nodes};
         ObsConsts k = obs_consts(c, c->step);
         for (int s = 0; s < nsteps; s++) {
             k.step = c->step + s;   // the state this step starts from
             launch_step_observed<S>(c, a, st);
-            obs_rows_reduce<<<parts, 32 * kObs, 0, st>>>(c->obs_rows, rows, partial, done, k, c->obs_series + s);
+            obs_rows_reduce<<<parts, kRowThreads, 0, st>>>(c->obs_rows, planes, rows, chunk, geo, partial, done, k,
+                                                          c->obs_series + s);
             c->swapped = !c->swapped;
             c->rest_phi = false;
             a.use_phi_fix = 0;
