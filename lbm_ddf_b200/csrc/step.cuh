@@ -1176,6 +1176,15 @@ __device__ __forceinline__ NodeOut<typename Codec<S>::R> update_node(const A &a,
     }
 }
 
+// For a launch that may start before the previous kernel of its stream is
+// done (programmatic dependent launch; passes at once without that
+// attribute): returns when that kernel has completed and its writes are
+// visible, so nothing before it may touch global memory.  The previous
+// kernel lets this one start as its blocks exit; letting it start earlier
+// puts its blocks into the slots a small grid leaves free, unevenly over the
+// SMs (B200, 32^3 FP64: 9.1 us per step against 5.9).
+__device__ __forceinline__ void await_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // One time step.  With OBS, the kernel also reduces the observables of the
 // state it reads — the moments every node update computes anyway — into one
 // row of FP64 sums per warp (row W b + w for warp w of block b, W =
@@ -1185,6 +1194,7 @@ template <class S, bool SWAPPED, bool PERIODIC, int COLL, bool OBS = false>
 __global__ void __launch_bounds__(bound_threads<S>(), step_threads_per_sm<S>() / bound_threads<S>())
     step_kernel(const StepArgs<S> a) {
     const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
+    await_previous();
     if constexpr (!OBS) {
         if (n >= a.nodes) return;
         update_node<S, SWAPPED, PERIODIC, COLL>(a, n);
