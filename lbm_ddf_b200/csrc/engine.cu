@@ -382,11 +382,35 @@ __global__ void import_pop_kernel(const StepArgs<S> a, int which, int k, const d
     });
 }
 
+// jy = sum c_y f, one population at a time in index order.
+__global__ void import_jy_kernel(const double *__restrict__ f, int sign, bool first, uint32_t nodes,
+                                 double *__restrict__ jy) {
+    const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= nodes) return;
+    const double j = first ? 0.0 : jy[n];
+    jy[n] = sign > 0 ? __dadd_rn(j, f[n]) : __dsub_rn(j, f[n]);
+}
+
+// Previous-step temperature from uy = sum(c_y f) + g*beta*(phi_prev - t0)/2.
+// For FP64 storage (exact) the estimate is nudged, one ulp at a time, until
+// the step's own formula, jy + 0.5*(gb*(phi_prev - t0)), gives back the
+// file's uy bit for bit, so the first step uses the velocity the reference
+// would use.
 template <class S>
-__global__ void import_phip_kernel(const StepArgs<S> a, const double *__restrict__ in) {
+__global__ void import_phip_kernel(const StepArgs<S> a, const double *__restrict__ uy, const double *__restrict__ jy,
+                                   double gb, double t0, bool exact) {
     const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= a.nodes) return;
-    a.phip[n] = (typename Codec<S>::P)in[n];
+    const double target = uy[n], j = jy[n];
+    double p = __dadd_rn(t0, __ddiv_rn(__dmul_rn(2.0, __dsub_rn(target, j)), gb));
+    if (exact && isfinite(p)) {
+        for (int it = 0; it < 64; it++) {
+            const double u = __dadd_rn(j, __dmul_rn(0.5, __dmul_rn(gb, __dsub_rn(p, t0))));
+            if (u == target) break;
+            p = nextafter(p, u < target ? INFINITY : -INFINITY);
+        }
+    }
+    a.phip[n] = (typename Codec<S>::P)p;
 }
 
 __device__ __forceinline__ uint64_t splitmix64(uint64_t x) {
@@ -951,47 +975,30 @@ int lbm_load_ref_state(lbm_case *c, const double *rho, const double *ux, const d
     if (!uy || !f || !g) return fail(LBM_ERR_ARG, "uy, f and g are required");
     DeviceGuard dg(c->p.device);
     const int64_t N = c->nodes;
-    // Previous-step temperature from uy = sum(c_y f) + g*beta*(phi_prev - t0)/2.
-    // For FP64 storage the estimate is nudged, one ulp at a time, until the
-    // device's own formula, jy + 0.5*(gb*(phi_prev - t0)), gives back the
-    // file's uy bit for bit, so the first step uses the velocity the
-    // reference would use.
-    std::vector<double> pp((size_t)N);
-    const double gb = c->p.gravity * c->p.beta;
-    const double t0 = c->d.t0;
-    const bool exact = c->p.storage == LBM_STORE_F64;
-    for (int64_t i = 0; i < N; i++) {
-        double jy = 0.0;
-        for (int k = 0; k < Q; k++) {
-            if (cy(k) > 0) jy += f[(size_t)k * N + i];
-            if (cy(k) < 0) jy -= f[(size_t)k * N + i];
-        }
-        double p = t0 + 2.0 * (uy[i] - jy) / gb;
-        if (exact && std::isfinite(p)) {
-            for (int it = 0; it < 64; it++) {
-                const volatile double h = gb * (p - t0);
-                const volatile double u = jy + 0.5 * h;
-                if (u == uy[i]) break;
-                p = std::nextafter(p, u < uy[i] ? INFINITY : -INFINITY);
-            }
-        }
-        pp[(size_t)i] = p;
-    }
+    // one population at a time through `stage`; sum(c_y f) gathers behind it
     double *stage = nullptr;
-    CUDA_TRY(cudaMalloc(&stage, (size_t)N * sizeof(double)));
+    CUDA_TRY(cudaMalloc(&stage, (size_t)N * 2 * sizeof(double)));
+    double *jy = stage + N;
+    const unsigned grid = grid_for(N, 256);
     rc = with_storage(c, [&](auto tag) {
         using S = std::remove_pointer_t<decltype(tag)>;
         const StepArgs<S> a = make_args<S>(c);
+        bool first = true;
         for (int which = 0; which < 2; which++)
             for (int k = 0; k < Q; k++) {
                 const double *src = (which ? g : f) + (size_t)k * N;
                 cudaError_t e = cudaMemcpy(stage, src, (size_t)N * sizeof(double), cudaMemcpyHostToDevice);
                 if (e != cudaSuccess) return fail(LBM_ERR_CUDA, cudaGetErrorString(e));
-                import_pop_kernel<S><<<grid_for(N, 256), 256>>>(a, which, k, stage);
+                import_pop_kernel<S><<<grid, 256>>>(a, which, k, stage);
+                if (which == 0 && cy(k) != 0) {
+                    import_jy_kernel<<<grid, 256>>>(stage, cy(k), first, a.nodes, jy);
+                    first = false;
+                }
             }
-        cudaError_t e = cudaMemcpy(stage, pp.data(), (size_t)N * sizeof(double), cudaMemcpyHostToDevice);
+        cudaError_t e = cudaMemcpy(stage, uy, (size_t)N * sizeof(double), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) return fail(LBM_ERR_CUDA, cudaGetErrorString(e));
-        import_phip_kernel<S><<<grid_for(N, 256), 256>>>(a, stage);
+        import_phip_kernel<S><<<grid, 256>>>(a, stage, jy, c->p.gravity * c->p.beta, c->d.t0,
+                                             c->p.storage == LBM_STORE_F64);
         return LBM_OK;
     });
     cudaError_t e = cudaDeviceSynchronize();
