@@ -807,8 +807,8 @@ __device__ __forceinline__ void store_word(const A &a, const Node &g, typename P
 // in the swapped one, against 664 and 652 with a node's update split over
 // two warps that exchanged their partial moments through shared memory (64
 // registers, 770-820 instructions per 32 nodes and a barrier; here ~550, no
-// barrier, and 27 loads in flight per warp instead of 13).  Closed box: 609
-// and 711 against 674 and 710.
+// barrier, and 27 loads in flight per warp instead of 13).  Closed box: 588
+// and 690 against 674 and 710.
 
 // The half of the opposite pairs that population k is summed in.  The
 // moments are two partial sums, added: the rest population and the pairs of
