@@ -221,8 +221,10 @@ __global__ void __launch_bounds__(kRowThreads) obs_rows_reduce(const double *__r
     for (int r = r0 + t / kObsRow; r < r1; r += 32) {
         const double v = rows[(size_t)r * kObsRow + word];
         s += v;
-        if (word == 5) {
-            const uint32_t first = 32u * (uint32_t)r, end = min(geo.nodes - 1u, first + 31u);
+        const uint32_t first = 32u * (uint32_t)r;
+        // (a warp past the last node wrote a row of zeros and no plane sums)
+        if (word == 5 && first < geo.nodes) {
+            const uint32_t end = min(geo.nodes - 1u, first + 31u);
             const uint32_t q0 = geo.div_lx.div(first), span = geo.div_lx.div(end) - q0;
             const int iy0 = (int)(q0 - geo.div_ly.div(q0) * (uint32_t)geo.ly);
             if (iy0 <= 2 || iy0 + (int)span >= geo.ly - 3) {
