@@ -117,6 +117,14 @@ __device__ __forceinline__ void finalize_observables(const double *__restrict__ 
 // 1072).
 template <class S> constexpr int kObsMinBlocks = 2;
 
+// Counts the calling block as done; true for the last of the grid.  The count
+// goes round the grid's size, so it is 0 again after every launch, and after
+// launches of one size that overlapped in spite of the header's rule, in
+// whatever order their blocks counted: no later launch finds it off.
+__device__ __forceinline__ bool counted_last(unsigned *done) {
+    return atomicInc(done, gridDim.x - 1) == gridDim.x - 1;
+}
+
 // Per-block partial sums, in FP64, of
 //   0 uy*phi  1 |u|^2  2 ux  3 uy  4 uz  5 phi
 //   6..8  phi on the planes iy = 0, 1, 2
@@ -126,7 +134,7 @@ template <class S> constexpr int kObsMinBlocks = 2;
 // 16-bit storage: the moments as the step of collision model `coll` forms
 // them, so these observables match those it reduces when it steps.
 //
-// With `done` (a count of finished blocks, 0 between launches) the block that
+// With `done` (a count of finished blocks, see counted_last) the block that
 // finishes last forms the observables too, so that reading a small case
 // costs one launch; `out` and `err_out`, the copy of the case's error flag,
 // may then be host memory the device can write, which saves the copies (B200,
@@ -179,14 +187,11 @@ __global__ void __launch_bounds__(kObsThreads, kObsMinBlocks<S>) obs_kernel(cons
     __shared__ bool last;
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
+    if (threadIdx.x == 0) last = counted_last(done);
     __syncthreads();
     if (!last) return;
     finalize_observables(partial, gridDim.x, consts, out);
-    if (threadIdx.x == 0) {
-        *done = 0u;
-        if (err_out) *err_out = *err;
-    }
+    if (threadIdx.x == 0 && err_out) *err_out = *err;
 }
 
 __global__ void __launch_bounds__(32 * kObs) obs_finalize(const double *__restrict__ partial, int nblocks,
@@ -201,7 +206,7 @@ __global__ void __launch_bounds__(32 * kObs) obs_finalize(const double *__restri
 // (coalesced); the phi thread also finds its rows' plane terms.  The 32 threads
 // of a term are then added in row order: a fixed order, so the result is
 // deterministic.  `done` counts the blocks that have written their partial
-// row; the last one resets it to 0 for the next launch.
+// row (counted_last).
 constexpr int kRowThreads = 32 * kObsRow;
 struct RowGeometry {
     FastDiv div_lx, div_ly;
@@ -247,11 +252,10 @@ __global__ void __launch_bounds__(kRowThreads) obs_rows_reduce(const double *__r
     }
     __threadfence();
     __syncthreads();
-    if (t == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
+    if (t == 0) last = counted_last(done);
     __syncthreads();
     if (!last) return;
     finalize_observables(partial, gridDim.x, c, out);
-    if (t == 0) *done = 0u;
 }
 
 // Vertical profile, src/output.cu:336-368: block b sums a chunk of the xz
@@ -710,7 +714,9 @@ template <class S> cudaError_t launch_step(const lbm_case *c, const StepArgs<S> 
 // `partial` and returns the blocks it ran: at most `cap` (the partial rows
 // there are) and at most the blocks `sms` SMs hold at once, so that the
 // grid-stride loop runs in one wave (8 blocks per SM asked of a kernel that
-// fits 5 would run a second, partly idle wave).
+// fits 5 would run a second, partly idle wave).  One number for both layouts
+// (the smaller; built for 2 blocks per SM they agree): all launches of a case
+// then have one grid, as counted_last asks.
 template <class S, bool SW, bool PER> int obs_resident() {
     static const int resident = [] {
         int n = 0;
@@ -727,9 +733,9 @@ template <class S, bool SW, bool PER> int obs_resident() {
 template <class S>
 int launch_obs(const lbm_case *c, const StepArgs<S> &a, double *partial, int cap, int sms, int coll, unsigned *done,
                const ObsConsts &k, lbm_observables *out, const int *err, int *err_out, cudaStream_t st) {
-    const bool per = c->p.sides == LBM_SIDES_PERIODIC;
-    const int resident = c->swapped ? (per ? obs_resident<S, true, true>() : obs_resident<S, true, false>())
-                                    : (per ? obs_resident<S, false, true>() : obs_resident<S, false, false>());
+    const int resident = c->p.sides == LBM_SIDES_PERIODIC
+                             ? std::min(obs_resident<S, true, true>(), obs_resident<S, false, true>())
+                             : std::min(obs_resident<S, true, false>(), obs_resident<S, false, false>());
     const int blocks = std::max(1, std::min(cap, sms * resident));
     LBM_DISPATCH_LAYOUT(c, obs_kernel, blocks, kObsThreads, st, a, partial, coll, done, k, out, err, err_out);
     return blocks;
