@@ -809,6 +809,15 @@ int check_case(const lbm_case *c, bool need_state) {
     return LBM_OK;
 }
 
+// Clears the error flag and the count of finished blocks of a case that has no
+// state yet, on the stream that gives it one: everything that reads them needs
+// a state, and so comes after.  (Cleared on another stream when the case is
+// created, they could still be as the allocation left them when a
+// non-blocking stream comes to read them.)
+cudaError_t clear_flags(const lbm_case *c, cudaStream_t st) {
+    return c->initialised ? cudaSuccess : cudaMemsetAsync(c->d_err, 0, 2 * sizeof(int), st);
+}
+
 // Calls that change a case's state or layout: not while it is a batch
 // member (the batch's descriptors and captured graphs describe its layout).
 int check_mutable(const lbm_case *c, bool need_state) {
@@ -882,7 +891,6 @@ int lbm_create(const lbm_params *p, lbm_case **out) {
     if (e == cudaSuccess) {
         c->d_err = (int *)((char *)c->partial + rows);
         c->obs_done = (unsigned *)(c->d_err + 1);
-        e = cudaMemset(c->d_err, 0, 2 * sizeof(int));
     }
     if (e == cudaSuccess) e = take_record(&c->host);
     if (e != cudaSuccess) {
@@ -919,6 +927,7 @@ static int init_common(lbm_case *c, int mode, uint64_t seed, double amplitude, v
     if (rc) return rc;
     DeviceGuard dg(c->p.device);
     cudaStream_t st = (cudaStream_t)stream;
+    CUDA_TRY(clear_flags(c, st));
     const uint64_t key = [&] {
         uint64_t x = seed + 0x9E3779B97F4A7C15ull;
         x = (x ^ (x >> 30)) * 0xBF58476D1CE4E5B9ull;
@@ -983,6 +992,7 @@ int lbm_load_ref_state(lbm_case *c, const double *rho, const double *ux, const d
     if (!uy || !f || !g) return fail(LBM_ERR_ARG, "uy, f and g are required");
     DeviceGuard dg(c->p.device);
     const int64_t N = c->nodes;
+    CUDA_TRY(clear_flags(c, nullptr));
     // one population at a time through `stage`; sum(c_y f) gathers behind it
     double *stage = nullptr;
     CUDA_TRY(cudaMalloc(&stage, (size_t)N * 2 * sizeof(double)));
@@ -1317,6 +1327,7 @@ int lbm_restore_state(lbm_case *c, const void *host, uint64_t bytes, void *strea
     DeviceGuard dg(c->p.device);
     cudaStream_t st = (cudaStream_t)stream;
     const char *b = (const char *)host;
+    CUDA_TRY(clear_flags(c, st));
     if (interleaved(c)) {
         CUDA_TRY(cudaMemcpyAsync(c->f, b + of, 2 * pb, cudaMemcpyHostToDevice, st));
     } else {
