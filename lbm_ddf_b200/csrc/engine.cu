@@ -742,50 +742,88 @@ int launch_obs(const lbm_case *c, const StepArgs<S> &a, double *partial, int cap
 }
 
 // Page-locked host records of the live cases, in pages of 32 (allocating and
-// freeing one costs ~0.6 ms, more than creating a small case).  A page whose
-// records are all back is freed unless it is the only one, so beyond one page
-// the memory follows the number of live cases.
+// freeing one costs 0.6 to 2 ms, more than creating a small case).  A page
+// belongs to the CUDA context it was allocated in, by that context's id, which
+// is never given twice: after a reset of the device a page of the old context
+// is neither handed out nor freed (its memory went with the context, and its
+// address may be someone else's).  A page whose records are all back is freed
+// unless it is the only one of its context, so beyond one page the memory
+// follows the number of live cases.  The list has no destructor, so a case may
+// be destroyed by another static object's at the process's end.
 struct RecordPage {
     struct alignas(128) Slot {
         HostRecord rec;
     };
-    Slot *slots = nullptr;
-    uint32_t used = 0;   // bit i: slot i is taken
+    Slot *slots;
+    uint64_t context;
+    uint32_t used;   // bit i: slot i is taken
+    RecordPage *next;
 };
 constexpr int kPageSlots = 32;
-std::mutex g_records_mu;
-std::vector<RecordPage> g_records;
+struct Records {
+    std::mutex mu;
+    RecordPage *pages = nullptr;
+} g_records;
+static_assert(std::is_trivially_destructible<Records>::value, "the list must outlive every case");
 
-cudaError_t take_record(HostRecord **out) {
-    std::lock_guard<std::mutex> lk(g_records_mu);
-    for (RecordPage &p : g_records)
-        for (int i = 0; i < kPageSlots; i++)
-            if (!(p.used >> i & 1u)) {
-                p.used |= 1u << i;
-                *out = &p.slots[i].rec;
-                return cudaSuccess;
-            }
-    RecordPage p;
+// Id of the calling thread's current CUDA context (that of the case's device,
+// under DeviceGuard); 0 if it cannot be had, and then no page is shared.
+uint64_t context_id() {
+    using Get = int (*)(void *, unsigned long long *);
+    static const Get get = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<Get>(f);
+    }();
+    unsigned long long id = 0;
+    return get && get(nullptr, &id) == 0 ? id : 0;
+}
+
+cudaError_t take_record(lbm_case *c) {
+    Records &r = g_records;
+    std::lock_guard<std::mutex> lk(r.mu);
+    c->context = context_id();
+    if (c->context)
+        for (RecordPage *p = r.pages; p; p = p->next)
+            for (int i = 0; p->context == c->context && i < kPageSlots; i++)
+                if (!(p->used >> i & 1u)) {
+                    p->used |= 1u << i;
+                    c->host = &p->slots[i].rec;
+                    return cudaSuccess;
+                }
+    RecordPage *p = new (std::nothrow) RecordPage{nullptr, c->context, 1u, r.pages};
+    if (!p) return cudaErrorMemoryAllocation;
     const cudaError_t e =
-        cudaHostAlloc((void **)&p.slots, kPageSlots * sizeof(RecordPage::Slot), cudaHostAllocPortable);
-    if (e != cudaSuccess) return e;
-    p.used = 1u;
-    *out = &p.slots[0].rec;
-    g_records.push_back(p);
+        cudaHostAlloc((void **)&p->slots, kPageSlots * sizeof(RecordPage::Slot), cudaHostAllocDefault);
+    if (e != cudaSuccess) {
+        delete p;
+        return e;
+    }
+    r.pages = p;
+    c->host = &p->slots[0].rec;
     return cudaSuccess;
 }
 
-void give_record(HostRecord *r) {
-    if (!r) return;
-    std::lock_guard<std::mutex> lk(g_records_mu);
-    for (size_t k = 0; k < g_records.size(); k++) {
-        RecordPage &p = g_records[k];
-        const auto *slot = reinterpret_cast<const RecordPage::Slot *>(r);
-        if (slot < p.slots || slot >= p.slots + kPageSlots) continue;
-        p.used &= ~(1u << (slot - p.slots));
-        if (p.used == 0 && g_records.size() > 1) {
-            cudaFreeHost(p.slots);
-            g_records.erase(g_records.begin() + (std::ptrdiff_t)k);
+void give_record(const lbm_case *c) {
+    if (!c->host) return;
+    const auto *slot = reinterpret_cast<const RecordPage::Slot *>(c->host);
+    Records &r = g_records;
+    std::lock_guard<std::mutex> lk(r.mu);
+    int pages = 0;
+    for (RecordPage *p = r.pages; p; p = p->next) pages += p->context == c->context;
+    for (RecordPage **at = &r.pages; *at; at = &(*at)->next) {
+        RecordPage *p = *at;
+        if (p->context != c->context || slot < p->slots || slot >= p->slots + kPageSlots) continue;
+        p->used &= ~(1u << (slot - p->slots));
+        if (p->used == 0 && (pages > 1 || !p->context)) {
+            if (p->context == context_id()) cudaFreeHost(p->slots);
+            *at = p->next;
+            delete p;
         }
         return;
     }
@@ -892,7 +930,7 @@ int lbm_create(const lbm_params *p, lbm_case **out) {
         c->d_err = (int *)((char *)c->partial + rows);
         c->obs_done = (unsigned *)(c->d_err + 1);
     }
-    if (e == cudaSuccess) e = take_record(&c->host);
+    if (e == cudaSuccess) e = take_record(c);
     if (e != cudaSuccess) {
         cudaGetLastError();
         lbm_destroy(c);
@@ -911,7 +949,7 @@ int lbm_destroy(lbm_case *c) {
     if (!interleaved(c)) cudaFree(c->g);
     cudaFree(c->phip);
     cudaFree(c->partial);
-    give_record(c->host);
+    give_record(c);
     cudaFree(c->prof);
     cudaFree(c->obs_rows);
     cudaFree(c->obs_series);

@@ -34,6 +34,7 @@ struct lbm_case {
     double *partial = nullptr;           // obs partial sums
     unsigned *obs_done = nullptr;        // blocks of the reduction that are done (behind partial)
     HostRecord *host = nullptr;          // what lbm_get_observables' kernel writes (page-locked)
+    uint64_t context = 0;                // id of the CUDA context `host` belongs to
     double *prof = nullptr;              // lbm_get_profile: chunk sums and the profile, from its first call
     int obs_blocks = 0;                  // partial rows (most reduction blocks)
     int sms = 148;                       // SM count of the case's device
