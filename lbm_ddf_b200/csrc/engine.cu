@@ -365,13 +365,15 @@ __global__ void export_macro_kernel(const StepArgs<S> a, double *__restrict__ ou
     out[4 * N + n] = (double)m.phi;
 }
 
-// Writes one population in the natural layout from FP64 values.
+// Writes one population of the nodes [first, end) in the natural layout from
+// their FP64 values.
 template <class S>
-__global__ void import_pop_kernel(const StepArgs<S> a, int which, int k, const double *__restrict__ in) {
+__global__ void import_pop_kernel(const StepArgs<S> a, int which, int k, uint32_t first, uint32_t end,
+                                  const double *__restrict__ in) {
     using C = Codec<S>;
-    const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= a.nodes) return;
-    const double v = in[n];
+    const uint32_t n = first + blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= end) return;
+    const double v = in[n - first];
     // 16-bit storage: shifted by the conduction profile at this node (natural layout)
     const uint32_t q = a.div_lx.div(n);
     const int iy = (int)(q - a.div_ly.div(q) * (uint32_t)a.ly);
@@ -403,11 +405,11 @@ __global__ void import_jy_kernel(const double *__restrict__ f, int sign, bool fi
 // file's uy bit for bit, so the first step uses the velocity the reference
 // would use.
 template <class S>
-__global__ void import_phip_kernel(const StepArgs<S> a, const double *__restrict__ uy, const double *__restrict__ jy,
-                                   double gb, double t0, bool exact) {
-    const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= a.nodes) return;
-    const double target = uy[n], j = jy[n];
+__global__ void import_phip_kernel(const StepArgs<S> a, uint32_t first, uint32_t end, const double *__restrict__ uy,
+                                   const double *__restrict__ jy, double gb, double t0, bool exact) {
+    const uint32_t n = first + blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= end) return;
+    const double target = uy[n - first], j = jy[n - first];
     double p = __dadd_rn(t0, __ddiv_rn(__dmul_rn(2.0, __dsub_rn(target, j)), gb));
     if (exact && isfinite(p)) {
         for (int it = 0; it < 64; it++) {
@@ -1031,33 +1033,48 @@ int lbm_load_ref_state(lbm_case *c, const double *rho, const double *ux, const d
     DeviceGuard dg(c->p.device);
     const int64_t N = c->nodes;
     CUDA_TRY(clear_flags(c, nullptr));
-    // one population at a time through `stage`; sum(c_y f) gathers behind it
+    // one population at a time through `stage`; sum(c_y f) gathers behind it.
+    // Where there is not the memory for both over all nodes, by quarters of
+    // the nodes.
     double *stage = nullptr;
-    CUDA_TRY(cudaMalloc(&stage, (size_t)N * 2 * sizeof(double)));
-    double *jy = stage + N;
-    const unsigned grid = grid_for(N, 256);
+    int64_t part = N;
+    cudaError_t e = cudaMalloc(&stage, (size_t)part * 2 * sizeof(double));
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        part = (N + 3) / 4;
+        e = cudaMalloc(&stage, (size_t)part * 2 * sizeof(double));
+    }
+    CUDA_TRY(e);
+    double *jy = stage + part;
     rc = with_storage(c, [&](auto tag) {
         using S = std::remove_pointer_t<decltype(tag)>;
         const StepArgs<S> a = make_args<S>(c);
-        bool first = true;
-        for (int which = 0; which < 2; which++)
-            for (int k = 0; k < Q; k++) {
-                const double *src = (which ? g : f) + (size_t)k * N;
-                cudaError_t e = cudaMemcpy(stage, src, (size_t)N * sizeof(double), cudaMemcpyHostToDevice);
-                if (e != cudaSuccess) return fail(LBM_ERR_CUDA, cudaGetErrorString(e));
-                import_pop_kernel<S><<<grid, 256>>>(a, which, k, stage);
-                if (which == 0 && cy(k) != 0) {
-                    import_jy_kernel<<<grid, 256>>>(stage, cy(k), first, a.nodes, jy);
-                    first = false;
+        for (int64_t first = 0; first < N; first += part) {
+            const int64_t count = std::min(part, N - first);
+            const uint32_t n0 = (uint32_t)first, n1 = (uint32_t)(first + count);
+            const unsigned grid = grid_for(count, 256);
+            auto upload = [&](const double *src) {
+                return cudaMemcpy(stage, src + first, (size_t)count * sizeof(double), cudaMemcpyHostToDevice);
+            };
+            bool none = true;
+            for (int which = 0; which < 2; which++)
+                for (int k = 0; k < Q; k++) {
+                    const cudaError_t e = upload((which ? g : f) + (size_t)k * N);
+                    if (e != cudaSuccess) return fail(LBM_ERR_CUDA, cudaGetErrorString(e));
+                    import_pop_kernel<S><<<grid, 256>>>(a, which, k, n0, n1, stage);
+                    if (which == 0 && cy(k) != 0) {
+                        import_jy_kernel<<<grid, 256>>>(stage, cy(k), none, (uint32_t)count, jy);
+                        none = false;
+                    }
                 }
-            }
-        cudaError_t e = cudaMemcpy(stage, uy, (size_t)N * sizeof(double), cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) return fail(LBM_ERR_CUDA, cudaGetErrorString(e));
-        import_phip_kernel<S><<<grid, 256>>>(a, stage, jy, c->p.gravity * c->p.beta, c->d.t0,
-                                             c->p.storage == LBM_STORE_F64);
+            const cudaError_t e = upload(uy);
+            if (e != cudaSuccess) return fail(LBM_ERR_CUDA, cudaGetErrorString(e));
+            import_phip_kernel<S><<<grid, 256>>>(a, n0, n1, stage, jy, c->p.gravity * c->p.beta, c->d.t0,
+                                                 c->p.storage == LBM_STORE_F64);
+        }
         return LBM_OK;
     });
-    cudaError_t e = cudaDeviceSynchronize();
+    e = cudaDeviceSynchronize();
     cudaFree(stage);
     if (rc) return rc;
     if (e != cudaSuccess) return fail(LBM_ERR_CUDA, cudaGetErrorString(e));
