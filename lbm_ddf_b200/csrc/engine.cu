@@ -206,16 +206,18 @@ __global__ void __launch_bounds__(32 * kObs) obs_finalize(const double *__restri
 // (coalesced); the phi thread also finds its rows' plane terms.  The 32 threads
 // of a term are then added in row order: a fixed order, so the result is
 // deterministic.  `done` counts the blocks that have written their partial
-// row (counted_last).
+// row (counted_last).  The rows are read through L2: the step that writes
+// them may still run when this kernel starts (await_previous), so they are
+// not constant memory for its whole life.
 constexpr int kRowThreads = 32 * kObsRow;
 struct RowGeometry {
     FastDiv div_lx, div_ly;
     int32_t ly;
     uint32_t nodes;
 };
-__global__ void __launch_bounds__(kRowThreads) obs_rows_reduce(const double *__restrict__ rows,
-                                                               const double *__restrict__ planes, int nrows, int chunk,
-                                                               RowGeometry geo, double *__restrict__ partial,
+__global__ void __launch_bounds__(kRowThreads) obs_rows_reduce(const double *rows, const double *planes, int nrows,
+                                                               int chunk, RowGeometry geo,
+                                                               double *__restrict__ partial,
                                                                unsigned *__restrict__ done, ObsConsts c,
                                                                lbm_observables *__restrict__ out) {
     __shared__ double red[kObs][32];
@@ -224,7 +226,7 @@ __global__ void __launch_bounds__(kRowThreads) obs_rows_reduce(const double *__r
     double s = 0.0, p[kObsPlanes] = {};
     await_previous();
     for (int r = r0 + t / kObsRow; r < r1; r += 32) {
-        const double v = rows[(size_t)r * kObsRow + word];
+        const double v = __ldcg(rows + (size_t)r * kObsRow + word);
         s += v;
         const uint32_t first = 32u * (uint32_t)r;
         // (a warp past the last node wrote a row of zeros and no plane sums)
@@ -235,7 +237,7 @@ __global__ void __launch_bounds__(kRowThreads) obs_rows_reduce(const double *__r
             if (iy0 <= 2 || iy0 + (int)span >= geo.ly - 3) {
 #pragma unroll
                 for (int k = 0; k < kObsPlanes; k++)
-                    p[k] += span ? planes[(size_t)r * kObsPlanes + k]
+                    p[k] += span ? __ldcg(planes + (size_t)r * kObsPlanes + k)
                                  : iy0 == (k < 3 ? k : geo.ly - 1 - (k - 3)) ? v : 0.0;
             }
         }
