@@ -294,8 +294,9 @@ int lbm_get_collision(const lbm_case *c, int32_t *model);
  * No counterpart in the reference, which runs one case per process.  A batch
  * holds cases (any grids, Ra, Pr) of one storage format, periodic sides, on
  * one device; it does not own them.  lbm_batch_step advances every member
- * by nsteps in one kernel launch per step (per about 150 members) (a CUDA graph of the launches is
- * captured on first use of a step count and replayed); each member's step
+ * by nsteps in one kernel launch per step, or a few launches for more than
+ * about 150 members (a CUDA graph of the launches is captured on first use of
+ * a step count and replayed); each member's step
  * count and layout advance as with lbm_step, and a member's result is the
  * same alone or in any mix; members may differ in collision model.  A case
  * belongs to at most one batch.  Members stay usable with the single-case

@@ -6,14 +6,16 @@
 // non-empty group (normally one: members move through the layouts in step;
 // more when a group has more members than one launch's parameters hold)
 // advances the group's members by one step.  Their nodes are cut into tiles
-// of BLOCK nodes, numbered case after case; one block per tile, or
-// BLOCKS_PER_SM x 148 persistent blocks walking the tile list with a grid
-// stride, finds each tile's case by a binary search over the tiles' prefix
-// sums in the kernel parameters, and applies the same node update as the
-// single-case kernel (step.cuh update_node) with that case's parameters.  A
-// kernel instance holds the code of one layout and one model only, so it
-// needs no more registers than the single-case kernel.  A case's result
-// does not depend on the other members.
+// of BLOCK nodes, numbered case after case; one block per tile finds the
+// tile's case by a binary search over the tiles' prefix sums in the kernel
+// parameters, and applies the same node update as the single-case kernel
+// (step.cuh update_node) with that case's parameters.  Persistent blocks
+// (BLOCKS_PER_SM x 148 of them walking the tile list with a grid stride) and
+// groups of very many small members take batch_table_kernel instead, which
+// finds the same in tables in global memory.  A kernel instance holds the
+// code of one layout and one model only, so it needs no more registers than
+// the single-case kernel.  A case's result does not depend on the other
+// members.
 //
 // Repeated steps are captured once into a CUDA graph (the launches of every
 // step, alternating layouts) and replayed.  The launch shape (block size and
@@ -97,35 +99,76 @@ template <class S, int MAX> struct BatchArgs {
 };
 
 // Members per launch: as many as the 32,764 bytes of kernel parameters hold,
-// or 32 (less to copy per launch).
+// or 32, for the smaller node of a captured graph (B200, capture and first
+// replay of 20 steps of two 32^3 cases, per step: 14 to 15 us, 22 with the
+// larger parameters; the replays alone are the same).
 template <class S> constexpr int batch_max() { return (32764 - 64) / (int)(sizeof(BatchCase<S>) + 4); }
 constexpr int kBatchSmall = 32;
+// A group of more members takes several launches per step, unless they are
+// small, with fewer nodes than this on average: then one launch of
+// batch_table_kernel.  B200, tables against parameters, us per step: 2000
+// cases of 16^3 FP64 1248 against 1322, FP16S regularised 501 against 517,
+// FP16S 476 against 462, and with a capture every 20 steps 1270 against 1457,
+// 511 against 619 and 486 against 569; 600 cases of 24^3 FP64 1260 against
+// 1170, FP16S 448 against 408, with a capture every 20 steps 1276 against 1246
+// and 457 against 460.
+constexpr int64_t kTableNodes = 8192;
 
 // Advances the members of one launch, all in layout SWAPPED and collision
 // model COLL, by one step.  A tile is BLOCK nodes of one member, one per
-// thread.  With WALK persistent blocks walk the tiles; without, a block has
-// one tile and so never loads behind its own stores, which is what the
-// single-case kernel owes its speed to (step.cuh).  B200, 16 FP32 serving
-// cases: 2064 us per step, as their single-case kernels, against 2289 with
-// tiles of four rounds, descriptors in global memory and prefix sums copied
-// to shared memory by every block.
-template <class S, int BLOCK, bool SWAPPED, int COLL, int MAX, bool WALK>
+// thread, and a block has one tile, so it never loads behind its own stores,
+// which is what the single-case kernel owes its speed to (step.cuh).  B200,
+// 16 FP32 serving cases: 2064 us per step, as their single-case kernels,
+// against 2289 with tiles of four rounds, descriptors in global memory and
+// prefix sums copied to shared memory by every block.
+template <class S, int BLOCK, bool SWAPPED, int COLL, int MAX>
 __global__ void __launch_bounds__(BLOCK, BatchOccupancy<S, BLOCK, COLL>::value)
     batch_step_kernel(const __grid_constant__ BatchArgs<S, MAX> b) {
-    const uint32_t end = b.start[b.n];
-    uint32_t t = blockIdx.x;
-    do {
-        int lo = 0, hi = b.n;   // the member c with start[c] <= t < start[c+1]
+    int lo = 0, hi = b.n;   // the member c with start[c] <= blockIdx.x < start[c+1]
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (b.start[mid] <= blockIdx.x) lo = mid;
+        else hi = mid;
+    }
+    const BatchCase<S> &cs = b.cases[lo];
+    const uint32_t u = (blockIdx.x - b.start[lo]) * BLOCK + threadIdx.x;
+    if (u < cs.nodes) update_node<S, SWAPPED, true, COLL>(cs, u);
+}
+
+// The same from tables in global memory, for the batches that
+// batch_step_kernel serves worse: persistent blocks, which look a member up
+// again for every tile, and very many small members (kTableNodes).  A tile is kTileRounds rounds of BLOCK nodes, so that the
+// lookup (prefix sums in shared memory, the descriptor in global memory) is
+// paid once for four nodes of a thread (B200, 32 FP32 cases at 8 blocks of 128
+// per SM: 3.49 ms per step, against 3.67 with one round and the tables in the
+// kernel parameters).  16-bit storage has the registers at which blocks that
+// load behind their own stores hide it best (32 FP16S cases: BGK 1.77 ms per
+// step at 512 threads per SM, 2.01 at 640; regularised 1.99 at 640, 2.06 at
+// 512, 2.13 at 768).
+constexpr int kTileRounds = 4;
+template <class S, int BLOCK, bool SWAPPED, int COLL>
+__global__ void __launch_bounds__(BLOCK, (sizeof(S) == 2 && COLL == LBM_COLLISION_REGULARIZED ? 640
+                                          : sizeof(S) == 2 ? 512 : step_threads_per_sm<S>()) / BLOCK)
+    batch_table_kernel(const BatchCase<S> *__restrict__ cases, int ncases, const uint32_t *__restrict__ tile_start) {
+    __shared__ uint32_t s_start[kMaxBatch + 1];
+    for (int i = threadIdx.x; i <= ncases; i += BLOCK) s_start[i] = tile_start[i];
+    __syncthreads();
+    const uint32_t end = s_start[ncases];
+    for (uint32_t t = s_start[0] + blockIdx.x; t < end; t += gridDim.x) {
+        int lo = 0, hi = ncases;
         while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
-            if (b.start[mid] <= t) lo = mid;
+            if (s_start[mid] <= t) lo = mid;
             else hi = mid;
         }
-        const BatchCase<S> &cs = b.cases[lo];
-        const uint32_t u = (t - b.start[lo]) * BLOCK + threadIdx.x;
-        if (u < cs.nodes) update_node<S, SWAPPED, true, COLL>(cs, u);
-        t += gridDim.x;
-    } while (WALK && t < end);
+        const BatchCase<S> &cs = cases[lo];
+        const uint32_t u0 = (t - s_start[lo]) * (BLOCK * kTileRounds) + threadIdx.x;
+#pragma unroll 1
+        for (int r = 0; r < kTileRounds; r++) {
+            const uint32_t u = u0 + r * BLOCK;
+            if (u < cs.nodes) update_node<S, SWAPPED, true, COLL>(cs, u);
+        }
+    }
 }
 
 }  // namespace lbm
@@ -141,9 +184,23 @@ struct lbm_batch {
     // from the batch's phase, bit 1 = regularised collision.  Every step
     // flips all layouts and the phase together, so groups stay fixed.
     int group_first[4] = {0, 0, 0, 0}, group_count[4] = {0, 0, 0, 0};
+    int64_t group_nodes[4] = {0, 0, 0, 0};
     int phase = 0;
     bool dirty = true;             // descriptors need rebuilding
     std::vector<unsigned char> h_cases;
+    // batch_table_kernel: device copies of the descriptors and of the tiles'
+    // prefix sums, and the page-locked staging of their uploads, two in turn:
+    // an upload is a copy on the step stream that needs no wait, and a staging
+    // buffer is reused only after its event says its copy is done
+    std::vector<uint32_t> h_start;
+    void *d_cases = nullptr;
+    uint32_t *d_start = nullptr;
+    int capacity = 0;
+    unsigned char *stage[2] = {nullptr, nullptr};
+    size_t stage_cap[2] = {0, 0};
+    cudaEvent_t stage_ev[2] = {nullptr, nullptr};
+    bool stage_used[2] = {false, false};
+    int stage_next = 0;
     // lbm_batch_observables: one record per member (device)
     lbm_observables *d_obs = nullptr;
     int obs_cap = 0;
@@ -224,8 +281,61 @@ int group_of(const lbm_batch *b, const lbm_case *c) {
     return ((c->swapped ? 1 : 0) ^ b->phase) | (c->collision == LBM_COLLISION_REGULARIZED ? 2 : 0);
 }
 
+// Whether the members of group g are stepped by batch_table_kernel.
+template <class S> bool by_table(const lbm_batch *b, int g) {
+    return b->launch == LBM_BATCH_TILES &&
+           (b->blocks_per_sm > 0 ||
+            (b->group_count[g] > batch_max<S>() && b->group_nodes[g] < kTableNodes * b->group_count[g]));
+}
+
+// Uploads the descriptors and the tiles' prefix sums for batch_table_kernel,
+// in stream order behind the steps already enqueued; the host does not wait.
+int upload_tables(lbm_batch *b, cudaStream_t st) {
+    const int n = (int)b->members.size();
+    const size_t db = case_desc_bytes(b->storage);
+    if (n > b->capacity) {
+        const int cap = std::max(n, std::max(16, 2 * b->capacity));
+        void *dc = nullptr;
+        uint32_t *ds = nullptr;
+        CUDA_TRY(cudaMalloc(&dc, (size_t)cap * db));
+        cudaError_t e = cudaMalloc(&ds, (size_t)(cap + 1) * sizeof(uint32_t));
+        if (e != cudaSuccess) {
+            cudaFree(dc);
+            return fail(LBM_ERR_NOMEM, "batch descriptor allocation failed");
+        }
+        CUDA_TRY(cudaStreamSynchronize(st));
+        cudaFree(b->d_cases);
+        cudaFree(b->d_start);
+        b->d_cases = dc;
+        b->d_start = ds;
+        b->capacity = cap;
+        drop_graphs(b);
+    }
+    const int i = b->stage_next;
+    const size_t cb = b->h_cases.size(), sb = b->h_start.size() * sizeof(uint32_t);
+    const size_t off = (cb + 255) / 256 * 256;
+    if (b->stage_used[i]) CUDA_TRY(cudaEventSynchronize(b->stage_ev[i]));
+    if (!b->stage_ev[i]) CUDA_TRY(cudaEventCreateWithFlags(&b->stage_ev[i], cudaEventDisableTiming));
+    if (b->stage_cap[i] < off + sb) {
+        if (b->stage[i]) cudaFreeHost(b->stage[i]);
+        b->stage[i] = nullptr;
+        b->stage_cap[i] = 0;
+        const size_t cap = std::max<size_t>(2 * (off + sb), 64 * 1024);
+        CUDA_TRY(cudaMallocHost((void **)&b->stage[i], cap));
+        b->stage_cap[i] = cap;
+    }
+    std::memcpy(b->stage[i], b->h_cases.data(), cb);
+    std::memcpy(b->stage[i] + off, b->h_start.data(), sb);
+    CUDA_TRY(cudaMemcpyAsync(b->d_cases, b->stage[i], cb, cudaMemcpyHostToDevice, st));
+    CUDA_TRY(cudaMemcpyAsync(b->d_start, b->stage[i] + off, sb, cudaMemcpyHostToDevice, st));
+    CUDA_TRY(cudaEventRecord(b->stage_ev[i], st));
+    b->stage_used[i] = true;
+    b->stage_next = 1 - i;
+    return LBM_OK;
+}
+
 // Rebuilds the descriptors after a membership change.
-int refresh(lbm_batch *b) {
+int refresh(lbm_batch *b, cudaStream_t st) {
     if (!b->dirty) return LBM_OK;
     const int n = (int)b->members.size();
     const size_t db = case_desc_bytes(b->storage);
@@ -233,34 +343,40 @@ int refresh(lbm_batch *b) {
     order.reserve((size_t)n);
     for (int g = 0; g < 4; g++) {
         b->group_first[g] = (int)order.size();
+        b->group_nodes[g] = 0;
         for (const lbm_case *c : b->members)
-            if (group_of(b, c) == g) order.push_back(c);
+            if (group_of(b, c) == g) {
+                order.push_back(c);
+                b->group_nodes[g] += c->nodes;
+            }
         b->group_count[g] = (int)order.size() - b->group_first[g];
     }
     b->h_cases.assign((size_t)n * db, 0);
+    b->h_start.assign((size_t)n + 1, 0);
+    bool tables = false;
     int rc = with_batch_storage(b, [&](auto tag) {
         using S = std::remove_pointer_t<decltype(tag)>;
         for (int i = 0; i < n; i++) {
             const BatchCase<S> d = describe<S>(order[(size_t)i]);
             std::memcpy(b->h_cases.data() + (size_t)i * db, &d, db);
+            const int64_t tile = (int64_t)b->block * kTileRounds;
+            b->h_start[i + 1] = b->h_start[i] + (uint32_t)((order[(size_t)i]->nodes + tile - 1) / tile);
         }
+        for (int g = 0; g < 4; g++) tables = tables || (b->group_count[g] > 0 && by_table<S>(b, g));
         return LBM_OK;
     });
+    if (rc == LBM_OK && tables) rc = upload_tables(b, st);
     if (rc) return rc;
     b->dirty = false;
     return LBM_OK;
 }
 
-unsigned grid_of(const lbm_batch *b, uint32_t tiles) {
-    if (b->blocks_per_sm <= 0) return tiles;
-    return (unsigned)std::min<uint64_t>(tiles, (uint64_t)b->sm_count * b->blocks_per_sm);
-}
-
 // One step of members [0, n) of one group (their descriptors at `d`), in
 // launches of at most MAX members.
 template <class S, int BLOCK, bool SW, int MAX>
-void launch_members(const lbm_batch *b, const unsigned char *d, int n, bool reg, cudaStream_t st) {
-    auto args = std::make_unique<BatchArgs<S, MAX>>();
+int launch_members(const unsigned char *d, int n, bool reg, cudaStream_t st) {
+    const std::unique_ptr<BatchArgs<S, MAX>> args(new (std::nothrow) BatchArgs<S, MAX>());
+    if (!args) return fail(LBM_ERR_NOMEM, "host allocation failed");
     for (int first = 0; first < n; first += MAX) {
         args->n = std::min(MAX, n - first);
         uint32_t tiles = 0;
@@ -270,25 +386,29 @@ void launch_members(const lbm_batch *b, const unsigned char *d, int n, bool reg,
             tiles += (args->cases[i].nodes + BLOCK - 1) / BLOCK;
         }
         args->start[args->n] = tiles;
-        auto launch = [&](auto walk) {
-            constexpr bool W = decltype(walk)::value;
-            const unsigned grid = grid_of(b, tiles);
-            if (reg) batch_step_kernel<S, BLOCK, SW, LBM_COLLISION_REGULARIZED, MAX, W><<<grid, BLOCK, 0, st>>>(*args);
-            else batch_step_kernel<S, BLOCK, SW, LBM_COLLISION_BGK, MAX, W><<<grid, BLOCK, 0, st>>>(*args);
-        };
-        if constexpr (MAX == batch_max<S>()) {
-            if (b->blocks_per_sm > 0) {
-                launch(std::true_type{});
-                continue;
-            }
-        }
-        launch(std::false_type{});
+        if (reg) batch_step_kernel<S, BLOCK, SW, LBM_COLLISION_REGULARIZED, MAX><<<tiles, BLOCK, 0, st>>>(*args);
+        else batch_step_kernel<S, BLOCK, SW, LBM_COLLISION_BGK, MAX><<<tiles, BLOCK, 0, st>>>(*args);
     }
+    return LBM_OK;
 }
-template <class S, int BLOCK, bool SW>
-void launch_group(const lbm_batch *b, const unsigned char *d, int n, bool reg, cudaStream_t st) {
-    if (n <= kBatchSmall && b->blocks_per_sm <= 0) launch_members<S, BLOCK, SW, kBatchSmall>(b, d, n, reg, st);
-    else launch_members<S, BLOCK, SW, batch_max<S>()>(b, d, n, reg, st);
+
+// One step of the members of group g, in layout SW.
+template <class S, int BLOCK, bool SW> int launch_group(const lbm_batch *b, int g, cudaStream_t st) {
+    const int n = b->group_count[g], first = b->group_first[g];
+    const bool reg = (g & 2) != 0;
+    if (by_table<S>(b, g)) {
+        const uint32_t *start = b->d_start + first;
+        const BatchCase<S> *cases = (const BatchCase<S> *)b->d_cases + first;
+        uint32_t grid = b->h_start[first + n] - b->h_start[first];
+        if (b->blocks_per_sm > 0)
+            grid = (uint32_t)std::min<uint64_t>(grid, (uint64_t)b->sm_count * b->blocks_per_sm);
+        if (reg) batch_table_kernel<S, BLOCK, SW, LBM_COLLISION_REGULARIZED><<<grid, BLOCK, 0, st>>>(cases, n, start);
+        else batch_table_kernel<S, BLOCK, SW, LBM_COLLISION_BGK><<<grid, BLOCK, 0, st>>>(cases, n, start);
+        return LBM_OK;
+    }
+    const unsigned char *d = b->h_cases.data() + (size_t)first * sizeof(BatchCase<S>);
+    return n <= kBatchSmall ? launch_members<S, BLOCK, SW, kBatchSmall>(d, n, reg, st)
+                            : launch_members<S, BLOCK, SW, batch_max<S>()>(d, n, reg, st);
 }
 
 // Lane of each member for the per-case launch: members by decreasing node
@@ -351,18 +471,13 @@ int enqueue_steps(lbm_batch *b, int nsteps, cudaStream_t st) {
         using S = std::remove_pointer_t<decltype(tag)>;
         for (int s = 0; s < nsteps; s++)
             for (int g = 0; g < 4; g++) {
-                const int n = b->group_count[g];
-                if (n == 0) continue;
-                const unsigned char *d = b->h_cases.data() + (size_t)b->group_first[g] * sizeof(BatchCase<S>);
+                if (b->group_count[g] == 0) continue;
                 const bool sw = ((g & 1) ^ b->phase ^ (s & 1)) != 0;
-                const bool reg = (g & 2) != 0;
-                if (b->block == 256) {
-                    if (sw) launch_group<S, 256, true>(b, d, n, reg, st);
-                    else launch_group<S, 256, false>(b, d, n, reg, st);
-                } else {
-                    if (sw) launch_group<S, 128, true>(b, d, n, reg, st);
-                    else launch_group<S, 128, false>(b, d, n, reg, st);
-                }
+                const int rc = b->block == 256 ? (sw ? launch_group<S, 256, true>(b, g, st)
+                                                     : launch_group<S, 256, false>(b, g, st))
+                                               : (sw ? launch_group<S, 128, true>(b, g, st)
+                                                     : launch_group<S, 128, false>(b, g, st));
+                if (rc) return rc;
             }
         return LBM_OK;
     });
@@ -416,12 +531,21 @@ int lbm_batch_destroy(lbm_batch *b) {
     for (lbm_case *m : b->members) m->batch = nullptr;
     DeviceGuard dg(b->device);
     drop_graphs(b);
+    cudaFree(b->d_cases);
+    cudaFree(b->d_start);
     cudaFree(b->d_obs);
     for (int l = 0; l < kLanes; l++) {
         if (b->lanes[l]) cudaStreamDestroy(b->lanes[l]);
         if (b->join_ev[l]) cudaEventDestroy(b->join_ev[l]);
     }
     if (b->fork_ev) cudaEventDestroy(b->fork_ev);
+    for (int i = 0; i < 2; i++) {
+        if (b->stage_ev[i]) {
+            cudaEventSynchronize(b->stage_ev[i]);
+            cudaEventDestroy(b->stage_ev[i]);
+        }
+        if (b->stage[i]) cudaFreeHost(b->stage[i]);
+    }
     if (b->capture_stream) cudaStreamDestroy(b->capture_stream);
     delete b;
     return LBM_OK;
@@ -472,6 +596,7 @@ int lbm_batch_set_config(lbm_batch *b, int32_t block, int32_t blocks_per_sm, int
     if (!b) return fail(LBM_ERR_ARG, "batch is NULL");
     if (block != 128 && block != 256) return fail(LBM_ERR_ARG, "block must be 128 or 256");
     if (blocks_per_sm < 0 || blocks_per_sm > 64) return fail(LBM_ERR_ARG, "blocks_per_sm must be 0..64");
+    if (block != b->block || blocks_per_sm != b->blocks_per_sm) b->dirty = true;   // the tiles change, or who walks them
     b->block = block;
     b->blocks_per_sm = blocks_per_sm;
     b->use_graph = use_graph != 0;
@@ -482,7 +607,10 @@ int lbm_batch_set_config(lbm_batch *b, int32_t block, int32_t blocks_per_sm, int
 int lbm_batch_set_launch(lbm_batch *b, int32_t launch) {
     if (!b) return fail(LBM_ERR_ARG, "batch is NULL");
     if (launch != LBM_BATCH_TILES && launch != LBM_BATCH_PER_CASE) return fail(LBM_ERR_ARG, "unknown batch launch");
-    if (launch != b->launch) drop_graphs(b);
+    if (launch != b->launch) {
+        b->dirty = true;   // the tile walk may need its tables
+        drop_graphs(b);
+    }
     b->launch = launch;
     return LBM_OK;
 }
@@ -507,7 +635,7 @@ int lbm_batch_step(lbm_batch *b, int32_t nsteps, void *stream) {
     if (nsteps == 0 || b->members.empty()) return LBM_OK;
     DeviceGuard dg(b->device);
     cudaStream_t st = (cudaStream_t)stream;
-    int rc = refresh(b);
+    int rc = refresh(b, st);
     if (rc) return rc;
     if (b->use_graph && nsteps > 1) {
         const int key = 2 * nsteps + b->phase;
