@@ -201,6 +201,23 @@ template <bool PERIODIC> __device__ __forceinline__ bool yz_interior(const Node 
     return g.vym && g.vyp && (PERIODIC || (g.vzm && g.vzp));
 }
 
+// The lanes of the calling warp that hold a node: its nodes are consecutive
+// and start at a multiple of 32 in every kernel that updates nodes or forms
+// their moments.
+template <class A> __device__ __forceinline__ unsigned node_lanes(const A &a, const Node &g) {
+    const uint32_t left = a.nodes - (g.n & ~31u);
+    return left >= 32u ? 0xffffffffu : (1u << left) - 1u;
+}
+
+// Whether rows are whole warps, so that a warp's nodes share an x-row.
+template <class A> __device__ __forceinline__ bool whole_warps(const A &a) { return (a.lx & 31) == 0; }
+
+// Whether all nodes of the warp are `inner` (in rows of whole warps, whether
+// this one is: they all are or none).
+template <class A> __device__ __forceinline__ bool one_body(const A &a, const Node &g, bool inner) {
+    return whole_warps(a) ? inner : __all_sync(node_lanes(a, g), inner);
+}
+
 // The path of node g's update (the INTERIOR argument, see inside_t):
 // kRowInside for rows whose y and z neighbours are inside, kAllInside for
 // those of a closed box when no active lane of the warp lies at an x wall
@@ -1033,12 +1050,12 @@ template <class A, class Put> __device__ __forceinline__ void reg_relax(const A 
 // ---- one node ----
 
 // Moments of node g on the path INTERIOR, then (with STORE) its collision and
-// its stores.  all_in: whether the warp's lanes on this path have all their
-// neighbours inside (a closed box's rows; see Shift).
+// its stores.  fold: whether the BGK collision folds the node's shift, all its
+// neighbours being inside (see Shift).
 template <class S, bool SWAPPED, bool PERIODIC, int COLL, int INTERIOR, bool STORE, class A, class Sink>
-__device__ __forceinline__ Moments<float> update_path16(const A &a, const Node &g, bool all_in, const Sink &sink) {
+__device__ __forceinline__ Moments<float> update_path16(const A &a, const Node &g, bool fold, const Sink &sink) {
     const float phip = a.phip[g.n];
-    const bool folded = COLL == LBM_COLLISION_BGK && SWAPPED && (all_inside<INTERIOR, PERIODIC>() || all_in);
+    const bool folded = COLL == LBM_COLLISION_BGK && SWAPPED && (all_inside<INTERIOR, PERIODIC>() || fold);
     const Shift sh = {shift0(a, g), folded ? 0.f : (float)a.t_dy, folded ? (float)a.t_dy : 0.f};
     typename Pack16<S>::T w[Q];
     Unroll<0, Q>::run([&](auto kk) {
@@ -1091,12 +1108,26 @@ __device__ __forceinline__ Moments<float> update_path16(const A &a, const Node &
 // saves its warps the selects but competes for the instruction cache (B200,
 // closed-box swapped step, BGK: 701 us at 256^3 FP16S with two bodies, 717
 // with three; 152 against 162 at 192x96x192 BF16S).
+//
+// With periodic sides a warp takes one body, the tested one if any of its
+// nodes needs it (rows that are not whole warps): a warp that took both would
+// wait for two rounds of loads and run twice the instructions (B200, two cases
+// of 16^3 FP16S on their own kernels: 3.7 us per step, 4.7 with both).  In a
+// closed box the tested body would have to fold too, and its spills cost the
+// whole warps more (85 to 96 us per step at 128^3 BF16S).
 template <class S, bool SWAPPED, bool PERIODIC, int COLL, bool STORE, class A, class Sink>
 __device__ __forceinline__ Moments<float> update_node16(const A &a, const Node &g, const Sink &sink) {
-    const int path = node_path<PERIODIC, SWAPPED>(g);
-    if (path != kNoneInside)
-        return update_path16<S, SWAPPED, PERIODIC, COLL, kRowInside, STORE>(a, g, path == kAllInside, sink);
-    return update_path16<S, SWAPPED, PERIODIC, COLL, kNoneInside, STORE>(a, g, false, sink);
+    if constexpr (PERIODIC) {
+        const bool inner = yz_interior<PERIODIC>(g);
+        if (one_body(a, g, inner))
+            return update_path16<S, SWAPPED, PERIODIC, COLL, kRowInside, STORE>(a, g, inner, sink);
+        return update_path16<S, SWAPPED, PERIODIC, COLL, kNoneInside, STORE>(a, g, inner, sink);
+    } else {
+        const int path = node_path<PERIODIC, SWAPPED>(g);
+        if (path != kNoneInside)
+            return update_path16<S, SWAPPED, PERIODIC, COLL, kRowInside, STORE>(a, g, path == kAllInside, sink);
+        return update_path16<S, SWAPPED, PERIODIC, COLL, kNoneInside, STORE>(a, g, false, sink);
+    }
 }
 
 // The moments of node g exactly as the 16-bit step forms them, so observables
@@ -1138,8 +1169,11 @@ __device__ __forceinline__ NodeOut<typename Codec<S>::R> update_node(const A &a,
         return {update_node16<S, SWAPPED, PERIODIC, COLL, true>(a, g, sink), g.iy};
     } else if constexpr (sizeof(S) == 4 && COLL == LBM_COLLISION_REGULARIZED) {
         const Node g = make_node<PERIODIC>(a, n);
-        return {yz_interior<PERIODIC>(g) ? update_reg32<SWAPPED, PERIODIC, kRowInside>(a, g, sink)
-                                         : update_reg32<SWAPPED, PERIODIC, kNoneInside>(a, g, sink),
+        // bodies as in update_node16
+        const bool inner = yz_interior<PERIODIC>(g);
+        return {(PERIODIC ? one_body(a, g, inner) : inner)
+                    ? update_reg32<SWAPPED, PERIODIC, kRowInside>(a, g, sink)
+                    : update_reg32<SWAPPED, PERIODIC, kNoneInside>(a, g, sink),
                 g.iy};
     } else {
     using R = typename Codec<S>::R;
