@@ -626,9 +626,12 @@ template <class S, bool SW, bool PER, bool OBS = false>
 void launch_step_t(const lbm_case *c, const StepArgs<S> &a, cudaStream_t st, bool overlap) {
     constexpr int threads = node_threads<S>();
     const unsigned grid = grid_for(c->nodes, threads);
-    const auto kernel = c->collision == LBM_COLLISION_REGULARIZED
-                            ? &step_kernel<S, SW, PER, LBM_COLLISION_REGULARIZED, OBS>
-                            : &step_kernel<S, SW, PER, LBM_COLLISION_BGK, OBS>;
+    auto kernel = c->collision == LBM_COLLISION_REGULARIZED
+                      ? &step_kernel<S, SW, PER, LBM_COLLISION_REGULARIZED, OBS>
+                      : &step_kernel<S, SW, PER, LBM_COLLISION_BGK, OBS>;
+    if constexpr (sizeof(S) == 2 && !OBS)
+        if (c->collision == LBM_COLLISION_BGK && grid <= (unsigned)(c->sms * (kSmallGridThreadsPerSm / threads)))
+            kernel = &step_kernel<S, SW, PER, LBM_COLLISION_BGK, OBS, kSmallGridThreadsPerSm>;
     if (overlap) launch_overlapped(kernel, grid, threads, st, a);
     else kernel<<<grid, threads, 0, st>>>(a);
 }

@@ -615,6 +615,13 @@ template <class S> __host__ __device__ constexpr int node_threads() { return siz
 template <class S> __host__ __device__ constexpr int step_threads_per_sm() {
     return sizeof(S) == 8 ? 384 : sizeof(S) == 4 ? 512 : 768;
 }
+// The same for 16-bit BGK steps of grids that the device holds at once at that
+// number: registers that hide nothing there keep the 27 words and their update
+// free of spills, on whose length such a step's time depends (B200, us per
+// step, against 768: 16^3 FP16S 2.8 and 3.3, 32^3 3.2 and 3.3, two cases of
+// 16^3 on their own kernels in a batch 3.4 and 3.7; regularised steps, with
+// few spills, the same).
+constexpr int kSmallGridThreadsPerSm = 512;
 // The step kernel's launch bounds (FP32's are stated for blocks of 128, the
 // same register budget).
 template <class S> constexpr int bound_threads() { return sizeof(S) == 2 ? node_threads<S>() : 128; }
@@ -1224,8 +1231,8 @@ __device__ __forceinline__ void await_previous() { asm volatile("griddepcontrol.
 // row of FP64 sums per warp (row W b + w for warp w of block b, W =
 // node_threads / 32: the nodes [32 row, 32 row + 32)), at no extra read of
 // the populations.
-template <class S, bool SWAPPED, bool PERIODIC, int COLL, bool OBS = false>
-__global__ void __launch_bounds__(bound_threads<S>(), step_threads_per_sm<S>() / bound_threads<S>())
+template <class S, bool SWAPPED, bool PERIODIC, int COLL, bool OBS = false, int PER_SM = step_threads_per_sm<S>()>
+__global__ void __launch_bounds__(bound_threads<S>(), PER_SM / bound_threads<S>())
     step_kernel(const StepArgs<S> a) {
     const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
     await_previous();
