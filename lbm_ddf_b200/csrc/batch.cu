@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(BLOCK, BatchOccupancy<S, BLOCK, COLL>::value)
     }
     const BatchCase<S> &cs = b.cases[lo];
     const uint32_t u = (blockIdx.x - b.start[lo]) * BLOCK + threadIdx.x;
-    if (u < cs.nodes) update_node<S, SWAPPED, true, COLL>(cs, u);
+    if (u < cs.nodes) update_node<S, SWAPPED, true, COLL, true>(cs, u);
 }
 
 // The same from tables in global memory, for the batches that
@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(BLOCK, (sizeof(S) == 2 && COLL == LBM_COLLISIO
 #pragma unroll 1
         for (int r = 0; r < kTileRounds; r++) {
             const uint32_t u = u0 + r * BLOCK;
-            if (u < cs.nodes) update_node<S, SWAPPED, true, COLL>(cs, u);
+            if (u < cs.nodes) update_node<S, SWAPPED, true, COLL, true>(cs, u);
         }
     }
 }

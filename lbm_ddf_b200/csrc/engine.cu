@@ -115,7 +115,7 @@ __device__ __forceinline__ void finalize_observables(const double *__restrict__ 
 // ahead (B200, lbm_get_observables at 256^3: FP32 676 us natural and 638
 // swapped without a bound, 569 and 588 with; FP64 1320 and 1338, 1023 and
 // 1072).
-template <class S> constexpr int kObsMinBlocks = 2;
+constexpr int kObsMinBlocks = 2;
 
 // Counts the calling block as done; true for the last of the grid.  The count
 // goes round the grid's size, so it is 0 again after every launch, and after
@@ -143,10 +143,9 @@ __device__ __forceinline__ bool counted_last(unsigned *done) {
 // 32^3 FP32: 45 us per lbm_get_observables with a second launch and two
 // copies, 23 with neither).  Without, obs_finalize follows.
 template <class S, bool SWAPPED, bool PERIODIC>
-__global__ void __launch_bounds__(kObsThreads, kObsMinBlocks<S>) obs_kernel(const StepArgs<S> a, double *__restrict__ partial,
-                                                          int coll, unsigned *__restrict__ done, ObsConsts consts,
-                                                          lbm_observables *__restrict__ out, const int *err,
-                                                          int *err_out) {
+__global__ void __launch_bounds__(kObsThreads, kObsMinBlocks)
+    obs_kernel(const StepArgs<S> a, double *__restrict__ partial, int coll, unsigned *__restrict__ done,
+               ObsConsts consts, lbm_observables *__restrict__ out, const int *err, int *err_out) {
     using R = typename Codec<S>::R;
     double acc[kObs];
 #pragma unroll
@@ -265,11 +264,13 @@ __global__ void __launch_bounds__(kRowThreads) obs_rows_reduce(const double *row
 // chunks in order.  Enough chunks that the grid fills the device: one block
 // per plane left most of it idle (B200: 3.4 ms at 256^3 FP32 and 4.25 ms at
 // 512x256x512 FP16S, 0.61 and 1.25 now; a read of the state takes 0.56 and
-// 1.15).
+// 1.15).  16-bit storage, which loads one word where the others load two
+// values, is built for a third block per SM (512x256x512 FP16S, swapped layout
+// 1.34 ms against 1.61 with two; natural 1.27 with either).
 constexpr int kProf = 5;
 template <class S, bool SWAPPED, bool PERIODIC>
-__global__ void __launch_bounds__(kObsThreads, kObsMinBlocks<S> + (sizeof(S) == 2)) profile_kernel(const StepArgs<S> a, uint32_t chunks,
-                                                              double *__restrict__ partial) {
+__global__ void __launch_bounds__(kObsThreads, kObsMinBlocks + (sizeof(S) == 2 ? 1 : 0))
+    profile_kernel(const StepArgs<S> a, uint32_t chunks, double *__restrict__ partial) {
     using R = typename Codec<S>::R;
     const uint32_t iy = blockIdx.x / chunks, chunk = blockIdx.x - iy * chunks;
     double acc[kProf] = {0, 0, 0, 0, 0};
@@ -626,12 +627,16 @@ template <class S, bool SW, bool PER, bool OBS = false>
 void launch_step_t(const lbm_case *c, const StepArgs<S> &a, cudaStream_t st, bool overlap) {
     constexpr int threads = node_threads<S>();
     const unsigned grid = grid_for(c->nodes, threads);
-    auto kernel = c->collision == LBM_COLLISION_REGULARIZED
-                      ? &step_kernel<S, SW, PER, LBM_COLLISION_REGULARIZED, OBS>
-                      : &step_kernel<S, SW, PER, LBM_COLLISION_BGK, OBS>;
-    if constexpr (sizeof(S) == 2 && !OBS)
-        if (c->collision == LBM_COLLISION_BGK && grid <= (unsigned)(c->sms * (kSmallGridThreadsPerSm / threads)))
-            kernel = &step_kernel<S, SW, PER, LBM_COLLISION_BGK, OBS, kSmallGridThreadsPerSm>;
+    const bool small = grid <= (unsigned)(c->sms * (kSmallGridThreadsPerSm / threads));
+    const auto pick = [&](auto coll) {
+        constexpr int C = decltype(coll)::value;
+        if constexpr (has_small_step<S, PER, C, OBS>())
+            if (small) return &step_kernel<S, SW, PER, C, OBS, true>;
+        return &step_kernel<S, SW, PER, C, OBS>;
+    };
+    const auto kernel = c->collision == LBM_COLLISION_REGULARIZED
+                            ? pick(std::integral_constant<int, LBM_COLLISION_REGULARIZED>{})
+                            : pick(std::integral_constant<int, LBM_COLLISION_BGK>{});
     if (overlap) launch_overlapped(kernel, grid, threads, st, a);
     else kernel<<<grid, threads, 0, st>>>(a);
 }

@@ -417,7 +417,8 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __
 // moments on D3Q27).  rho, u and phi are unchanged, as in BGK; at tau = 1 the
 // two models coincide.  Every operation is an explicit round-to-nearest one,
 // so a case gives bitwise the same result in the single-case and the batch
-// kernels, in FP64 and FP32.
+// kernels.  FP64 steps run it; FP32 and 16-bit ones its operations on the
+// sums alone (reg_sums, reg_relax).
 template <class R>
 __device__ __forceinline__ void collide_reg(R (&fr)[Q], R (&gr)[Q], const Moments<R> &m, R omega_f, R omega_g,
                                             R force_fac, R gb, R t0) {
@@ -615,19 +616,25 @@ template <class S> __host__ __device__ constexpr int node_threads() { return siz
 template <class S> __host__ __device__ constexpr int step_threads_per_sm() {
     return sizeof(S) == 8 ? 384 : sizeof(S) == 4 ? 512 : 768;
 }
-// The same for 16-bit BGK steps of grids that the device holds at once at that
-// number: registers that hide nothing there keep the 27 words and their update
-// free of spills, on whose length such a step's time depends (B200, us per
-// step, against 768: 16^3 FP16S 2.8 and 3.3, 32^3 3.2 and 3.3, two cases of
-// 16^3 on their own kernels in a batch 3.4 and 3.7; regularised steps, with
-// few spills, the same).
+// Grids that the device holds at once at this many threads per SM have a step
+// of their own (SMALL below), whose time is the length of one update: 16-bit
+// BGK is built for this number, since registers that hide nothing there keep
+// the 27 words and their update free of spills (B200, us per step, against
+// 768: 16^3 FP16S 2.8 and 3.3, 32^3 3.2 and 3.3, two cases of 16^3 on their own
+// kernels in a batch 3.4 and 3.7; regularised steps, with few spills, the
+// same), and with periodic sides a warp runs one body (update_node16).
 constexpr int kSmallGridThreadsPerSm = 512;
+template <class S, bool PERIODIC, int COLL, bool OBS> constexpr bool has_small_step() {
+    return !OBS && ((sizeof(S) == 2 && (COLL == LBM_COLLISION_BGK || PERIODIC)) ||
+                    (sizeof(S) == 4 && COLL == LBM_COLLISION_REGULARIZED && PERIODIC));
+}
+template <class S, int COLL, bool SMALL> constexpr int step_budget() {
+    return SMALL && sizeof(S) == 2 && COLL == LBM_COLLISION_BGK ? kSmallGridThreadsPerSm : step_threads_per_sm<S>();
+}
 // The step kernel's launch bounds (FP32's are stated for blocks of 128, the
 // same register budget).
 template <class S> constexpr int bound_threads() { return sizeof(S) == 2 ? node_threads<S>() : 128; }
 
-// The whole update of one node: gather, moments, collision, carried
-// temperature, scatter.
 // ---- observables of a node's moments --------------------------------------
 //
 // FP64 sums of
@@ -1116,15 +1123,18 @@ __device__ __forceinline__ Moments<float> update_path16(const A &a, const Node &
 // closed-box swapped step, BGK: 701 us at 256^3 FP16S with two bodies, 717
 // with three; 152 against 162 at 192x96x192 BF16S).
 //
-// With periodic sides a warp takes one body, the tested one if any of its
-// nodes needs it (rows that are not whole warps): a warp that took both would
-// wait for two rounds of loads and run twice the instructions (B200, two cases
-// of 16^3 FP16S on their own kernels: 3.7 us per step, 4.7 with both).  In a
-// closed box the tested body would have to fold too, and its spills cost the
-// whole warps more (85 to 96 us per step at 128^3 BF16S).
-template <class S, bool SWAPPED, bool PERIODIC, int COLL, bool STORE, class A, class Sink>
+// With ONE_BODY (periodic sides) a warp takes one body, the tested one if any
+// of its nodes needs it (rows that are not whole warps): a warp that took both
+// would wait for two rounds of loads and run twice the instructions, which on
+// grids of small members and in small grids is most of the time (B200, two
+// cases of 16^3 FP16S on their own kernels: 3.7 us per step, 4.7 with both).
+// Large grids have few such warps and do better without the vote's registers
+// (ensemble of 32, 0.7%), and a closed box's tested body would have to fold
+// too, whose spills cost the whole warps more (85 to 96 us per step at 128^3
+// BF16S).  The results are the same, bit for bit.
+template <class S, bool SWAPPED, bool PERIODIC, int COLL, bool STORE, bool ONE_BODY, class A, class Sink>
 __device__ __forceinline__ Moments<float> update_node16(const A &a, const Node &g, const Sink &sink) {
-    if constexpr (PERIODIC) {
+    if constexpr (PERIODIC && ONE_BODY) {
         const bool inner = yz_interior<PERIODIC>(g);
         if (one_body(a, g, inner))
             return update_path16<S, SWAPPED, PERIODIC, COLL, kRowInside, STORE>(a, g, inner, sink);
@@ -1141,7 +1151,7 @@ __device__ __forceinline__ Moments<float> update_node16(const A &a, const Node &
 // reduced from them match those an observed step reduces.
 template <class S, bool SWAPPED, bool PERIODIC, int COLL, class A>
 __device__ __forceinline__ Moments<float> step_moments16(const A &a, const Node &g) {
-    return update_node16<S, SWAPPED, PERIODIC, COLL, false>(a, g, NoMomentSink{});
+    return update_node16<S, SWAPPED, PERIODIC, COLL, false, false>(a, g, NoMomentSink{});
 }
 
 // FP32 with the regularised collision, likewise: 54 values loaded, 18 sums
@@ -1168,17 +1178,17 @@ __device__ __forceinline__ Moments<float> update_reg32(const A &a, const Node &g
     return t.m;
 }
 
-template <class S, bool SWAPPED, bool PERIODIC, int COLL = LBM_COLLISION_BGK, class A, class Sink = NoMomentSink>
+template <class S, bool SWAPPED, bool PERIODIC, int COLL, bool ONE_BODY, class A, class Sink = NoMomentSink>
 __device__ __forceinline__ NodeOut<typename Codec<S>::R> update_node(const A &a, uint32_t n,
                                                                      const Sink &sink = Sink()) {
     if constexpr (sizeof(S) == 2) {
         const Node g = make_node<PERIODIC>(a, n);
-        return {update_node16<S, SWAPPED, PERIODIC, COLL, true>(a, g, sink), g.iy};
+        return {update_node16<S, SWAPPED, PERIODIC, COLL, true, ONE_BODY>(a, g, sink), g.iy};
     } else if constexpr (sizeof(S) == 4 && COLL == LBM_COLLISION_REGULARIZED) {
         const Node g = make_node<PERIODIC>(a, n);
         // bodies as in update_node16
         const bool inner = yz_interior<PERIODIC>(g);
-        return {(PERIODIC ? one_body(a, g, inner) : inner)
+        return {(PERIODIC && ONE_BODY ? one_body(a, g, inner) : inner)
                     ? update_reg32<SWAPPED, PERIODIC, kRowInside>(a, g, sink)
                     : update_reg32<SWAPPED, PERIODIC, kNoneInside>(a, g, sink),
                 g.iy};
@@ -1231,14 +1241,14 @@ __device__ __forceinline__ void await_previous() { asm volatile("griddepcontrol.
 // row of FP64 sums per warp (row W b + w for warp w of block b, W =
 // node_threads / 32: the nodes [32 row, 32 row + 32)), at no extra read of
 // the populations.
-template <class S, bool SWAPPED, bool PERIODIC, int COLL, bool OBS = false, int PER_SM = step_threads_per_sm<S>()>
-__global__ void __launch_bounds__(bound_threads<S>(), PER_SM / bound_threads<S>())
+template <class S, bool SWAPPED, bool PERIODIC, int COLL, bool OBS = false, bool SMALL = false>
+__global__ void __launch_bounds__(bound_threads<S>(), step_budget<S, COLL, SMALL>() / bound_threads<S>())
     step_kernel(const StepArgs<S> a) {
     const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
     await_previous();
     if constexpr (!OBS) {
         if (n >= a.nodes) return;
-        update_node<S, SWAPPED, PERIODIC, COLL>(a, n);
+        update_node<S, SWAPPED, PERIODIC, COLL, SMALL>(a, n);
     } else {
         using T = typename Codec<S>::R;
         constexpr int kT = node_threads<S>();
@@ -1250,7 +1260,7 @@ __global__ void __launch_bounds__(bound_threads<S>(), PER_SM / bound_threads<S>(
         const bool valid = n < a.nodes;
         if (valid) {
             volatile T *mine = &parked[0][threadIdx.x];
-            iy = update_node<S, SWAPPED, PERIODIC, COLL>(a, n, SharedMomentSink<T, kT>{mine}).iy;
+            iy = update_node<S, SWAPPED, PERIODIC, COLL, SMALL>(a, n, SharedMomentSink<T, kT>{mine}).iy;
             const double ux = mine[0], uy = mine[kT], uz = mine[2 * kT], phi = mine[3 * kT], rho = mine[4 * kT];
             d[0] = uy * phi;
             d[1] = ux * ux + uy * uy + uz * uz;
