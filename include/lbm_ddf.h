@@ -123,10 +123,12 @@ int lbm_derive(const lbm_params *p, lbm_derived *out);
  * temperature, reduction scratch), for admission against a memory budget.
  * The first lbm_step_observed call adds the rows of its in-kernel reduction
  * (14 doubles per 32 nodes, under 4 bytes per node) and one lbm_observables
- * per step of the longest call made; the first lbm_get_profile call adds at
- * most 40 bytes per plane and 100 KB.  A case also holds a record of page-locked
- * host memory, which lbm_get_observables' kernel writes; the library keeps
- * them in pages of 4 KB, one of which it never frees. */
+ * per step of the longest call made; the first lbm_get_profile call adds less
+ * than 80 bytes per plane and 640 bytes per SM.  A case also holds a record of
+ * page-locked host memory, which lbm_get_observables' kernel writes; the
+ * library keeps them in pages of 4 KB, one of which it does not free while its
+ * CUDA context lives.  lbm_load_ref_state takes 16 bytes per node while it
+ * runs, or 4 where there is no room for them. */
 int lbm_case_bytes(const lbm_params *p, uint64_t *bytes);
 
 /* Allocates a case on p->device (replaces the cudaMalloc calls of
@@ -330,8 +332,8 @@ int lbm_batch_observables(lbm_batch *b, lbm_observables *out, void *stream);
 int lbm_batch_set_config(lbm_batch *b, int32_t block, int32_t blocks_per_sm, int32_t use_graph);
 int lbm_batch_get_config(const lbm_batch *b, int32_t *block, int32_t *blocks_per_sm, int32_t *use_graph);
 /* How a batch step is launched.  LBM_BATCH_TILES (the default): one
- * persistent kernel per group of members walks every member's tiles (the
- * launch shape above).  LBM_BATCH_PER_CASE: each member's own single-case
+ * kernel per group of members steps every member's tiles (the launch shape
+ * above).  LBM_BATCH_PER_CASE: each member's own single-case
  * step kernel (the one lbm_step launches, its parameters in the constant
  * bank), the members spread over 8 streams forked from and joined to the
  * batch's stream, so in a captured graph they run as parallel branches;

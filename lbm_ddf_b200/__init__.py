@@ -452,7 +452,7 @@ class Case:
 
 
 class Batch:
-    """Cases advanced together by one kernel launch per step (C ABI
+    """Cases advanced together by one kernel launch per step, or a few (C ABI
     lbm_batch_*).  The batch does not own its cases."""
 
     def __init__(self, storage=STORE_F32, device: int = 0):
@@ -522,9 +522,9 @@ class Batch:
         check(lib().lbm_batch_set_config(self._h, block, blocks_per_sm, int(bool(use_graph))))
 
     def set_launch(self, launch):
-        """'tiles' (one persistent kernel walks every member's tiles; the
-        default) or 'per_case' (each member's own single-case kernel, the
-        members on parallel streams)."""
+        """'tiles' (one kernel steps every member's tiles; the default) or
+        'per_case' (each member's own single-case kernel, the members on
+        parallel streams)."""
         check(lib().lbm_batch_set_launch(self._h, BATCH_LAUNCH_NAMES.get(launch, launch)))
 
     @property

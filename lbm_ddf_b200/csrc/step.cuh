@@ -603,8 +603,8 @@ __device__ __forceinline__ void scatter(const A &a, const Node &g, const typenam
 // Threads per block of step_kernel: FP32 and 16-bit steps in blocks of two
 // warps (a block holds its SM slot until its slowest warp is done, and
 // two-warp blocks waste less of it: B200, 256^3 FP32, natural layout -1.8%,
-// closed-box swapped -3.6%; FP16S BGK closed-box swapped 640 against 667 for
-// the pair of layouts); FP64 measured 3% slower so and keeps four.
+// closed-box swapped -3.6%; FP16S BGK closed box -4% over both layouts); FP64
+// measured 3% slower so and keeps four.
 template <class S> __host__ __device__ constexpr int node_threads() { return sizeof(S) == 8 ? 128 : 64; }
 // Resident threads per SM the register allocation is sized for: 384 (<= 168
 // registers) for FP64, which holds 54 doubles across the collision (B200,
@@ -929,8 +929,8 @@ __device__ __forceinline__ void bgk_relax_store(const A &a, const Node &g, const
     };
     relax(std::integral_constant<int, 0>{}, -0.5f * uv);
     // corners, edges, faces: of the orders tried, the one whose registers
-    // spill least where it costs (closed box, swapped layout: 706 us at 256^3
-    // FP16S and 150 at 192x96x192 BF16S, against 709 and 169 in index order)
+    // spill least where it costs (closed box, swapped layout: 0.4% less time at
+    // 256^3 FP16S and 11% less at 192x96x192 BF16S than in index order)
     auto pairs = [&](auto cls) {
         Unroll<1, Q>::run([&](auto ii) {
             constexpr int I = decltype(ii)::value;
@@ -1120,8 +1120,8 @@ __device__ __forceinline__ Moments<float> update_path16(const A &a, const Node &
 // box's rows take one body whether or not a warp holds an x-wall node, with
 // the x-moving addresses by a select: a third body for the warps without one
 // saves its warps the selects but competes for the instruction cache (B200,
-// closed-box swapped step, BGK: 701 us at 256^3 FP16S with two bodies, 717
-// with three; 152 against 162 at 192x96x192 BF16S).
+// closed-box swapped step, BGK: 2% more time at 256^3 FP16S with three bodies,
+// 6% at 192x96x192 BF16S).
 //
 // With ONE_BODY (periodic sides) a warp takes one body, the tested one if any
 // of its nodes needs it (rows that are not whole warps): a warp that took both
@@ -1147,8 +1147,9 @@ __device__ __forceinline__ Moments<float> update_node16(const A &a, const Node &
     }
 }
 
-// The moments of node g exactly as the 16-bit step forms them, so observables
-// reduced from them match those an observed step reduces.
+// The moments of node g as the 16-bit step forms them (a closed box's rows by
+// the vote that the step takes over the same nodes), so observables reduced
+// from them match those an observed step reduces.
 template <class S, bool SWAPPED, bool PERIODIC, int COLL, class A>
 __device__ __forceinline__ Moments<float> step_moments16(const A &a, const Node &g) {
     return update_node16<S, SWAPPED, PERIODIC, COLL, false, false>(a, g, NoMomentSink{});

@@ -2,9 +2,9 @@
 
 Requests (grid, Ra, Pr, step budget, storage) arrive as a Poisson stream.
 The server keeps every admitted case resident in HBM and advances all of
-them together: one batch per storage format (lbm_batch_*), one kernel launch
-per step covering every resident case, replayed from CUDA graphs in chunks
-of `obs_every` steps.  Each chunk also enqueues the observables of every
+them together: one batch per storage format (lbm_batch_*), stepped by one
+kernel launch per about 150 resident cases, replayed from CUDA graphs in
+chunks of `obs_every` steps.  Each chunk also enqueues the observables of every
 member (lbm_batch_observables: one asynchronous copy per batch), and the
 next chunk is enqueued before the host reads them, so the device does not
 wait for the host between chunks.  The host then records each case's Nu time
